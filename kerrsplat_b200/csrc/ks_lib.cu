@@ -164,62 +164,164 @@ __device__ void gl_panel(const RayCT<T>& R, const MarchRay<T>& M, TimeT<T> ta, T
 
 constexpr int kAnchorPanelSamples = 4;
 
-__global__ void k_anchor_segments(Spacetime st, const double* __restrict__ alpha, const double* __restrict__ beta,
-                                  const long long* __restrict__ perm, long long npix, long long npad, const double* __restrict__ f,
-                                  const long long* __restrict__ aoff, double* __restrict__ anchors) {
-    long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int m = blockIdx.y;
-    if (j >= npix) return;
-    int nanch = int(f[PF_NANCH * npad + j]);
-    if (m >= nanch) return;
-    long long i = perm[j];
-    RayC R = build_ray(st, alpha[i], beta[i]);
-    int Man = int(f[PF_MANCHOR * npad + j]);
-    double dtau = f[PF_DTAU * npad + j];
-    MarchRay<double> M = march_ray_of(R, st, dtau);
-    int k = 1 + m * Man;
-    double tau = k * dtau;
-    double* A = anchors + (aoff[j] + m) * AF_COUNT;
-    JS<double> xr = xr_at(R, tau), xt = xt_at(R, tau);
-    A[AF_XR_SN] = xr.sn; A[AF_XR_CN] = xr.cn; A[AF_XR_DN] = xr.dn;
-    A[AF_XT_SN] = xt.sn; A[AF_XT_CN] = xt.cn; A[AF_XT_DN] = xt.dn;
-    double th, cth; bool nu;
-    polar_cos(M, xt, th, cth, nu);
-    bool ok = (tau <= R.tau_valid) && visible(M, cth);
-    A[AF_OK] = ok ? 1.0 : 0.0;
-    A[AF_PAD] = 0.0;
-    if (!(tau <= R.tau_valid)) {
-        A[AF_T] = 0.0; A[AF_PHI] = 0.0; A[AF_SEG_T] = 0.0; A[AF_SEG_PHI] = 0.0;
-        return;
-    }
-    // closed-form parts at tau, accumulated from the observer
-    Point<double> p = ray_point(M, xr, xt, tau);
-    double r = p.r;
-    double F = r + 2.0 * log(r);
-    double L = (R.scattering && tau > R.fo) ? F - 2.0 * (R.r4 + 2.0 * log(R.r4)) : -F;
-    double lp = log((r - st.rp) / r) / R.sp;
-    double lm = log((r - st.rmn) / r) / R.sm;
-    JS<double> x0 = xt_at(R, 0.0);
-    double sn0 = x0.sn / (R.pscale * x0.dn), cn0 = x0.cn / x0.dn;
-    A[AF_T] = L + R.Qt * lp + R.Qtm * lm;
-    A[AF_PHI] = R.Qphi * lp + R.Qphim * lm + polar_closed(M, tau, p.sn, p.cn) - polar_closed(M, 0.0, sn0, cn0);
-    // smooth part over (previous anchor, tau]
-    double ta = (m == 0) ? 0.0 : (1 + (m - 1) * Man) * dtau;
-    int nsamp = (m == 0) ? 1 : Man;
-    int np = (m == 0) ? 1 : (nsamp + kAnchorPanelSamples - 1) / kAnchorPanelSamples;
-    double hp = (tau - ta) / np;
-    double It = 0.0, Ip = 0.0;
-    for (int q = 0; q < np; ++q) {
-        double a0 = ta + q * hp, b0 = (q == np - 1) ? tau : ta + (q + 1) * hp;
-        double t1, p1;
-        if (R.scattering && a0 < R.fo && R.fo < b0) {
-            gl_panel(R, M, a0, R.fo, t1, p1); It += t1; Ip += p1;
-            gl_panel(R, M, R.fo, b0, t1, p1); It += t1; Ip += p1;
-        } else {
-            gl_panel(R, M, a0, b0, t1, p1); It += t1; Ip += p1;
+// The Landen scale of one modulus: the amplitude of any argument without the scale's square roots again.
+struct AmScale {
+    double ratio[12], top;
+    int n;
+    __device__ explicit AmScale(double m) {
+        double a = 1.0, b = sqrt(1.0 - m), c = sqrt(m);
+        n = 0;
+        while (n < 11 && c > kEps * a) {
+            const double a1 = 0.5 * (a + b);
+            c = c * c / (4.0 * a1);
+            b = sqrt(a * b);
+            a = a1;
+            ratio[n++] = c / a;
         }
+        top = ldexp(a, n);
     }
-    A[AF_SEG_T] = It; A[AF_SEG_PHI] = Ip;
+    __device__ JS<double> state(double u, double mu) const {
+        double ph = top * u;
+        for (int i = n - 1; i >= 0; --i) ph = 0.5 * (ph + asin(ratio[i] * sin(ph)));
+        double s, c;
+        sincos(ph, &s, &c);
+        return {s, c, sqrt(fma(-mu, s * s, 1.0))};
+    }
+};
+
+// jstep with one reciprocal
+__device__ __forceinline__ JS<double> jadd(const JS<double>& x, const JS<double>& d, double mu) {
+    const double inv = 1.0 / (1.0 - mu * (x.sn * x.sn) * (d.sn * d.sn));
+    return {(x.sn * d.cn * d.dn + d.sn * x.cn * x.dn) * inv, (x.cn * d.cn - x.sn * x.dn * d.sn * d.dn) * inv,
+            (x.dn * d.dn - mu * x.sn * x.cn * d.sn * d.cn) * inv};
+}
+
+// The per-ray factors of the smooth integrands (smooth() in their FP64 form) and the integrands at a pair
+// of Jacobi states: the horizon factors share one reciprocal, Delta = (r - r_+)(r - r_-), and cos theta
+// enters through its square only.
+struct AnchorRates {
+    double wpf, wmf, Q, qp, qpm, poln, ips;
+    __device__ AnchorRates(const MarchRay<double>& M)
+        : wpf(M.rp / M.sp), wmf(M.rmn / M.sm), Q(M.eta + (M.lam - M.a) * (M.lam - M.a)), qp(M.Qphi), qpm(M.Qphim), poln(M.lam * M.qC),
+          ips(1.0 / M.pscale) {}
+    __device__ void at(const MarchRay<double>& M, const JS<double>& xr, const JS<double>& xt, bool inbound, double& gt, double& gp) const {
+        const double a = M.a, lam = M.lam, r = radius(M, xr);
+        const double di = 1.0 / xt.dn, sn = xt.sn * di * ips, cn = xt.cn * di, sn2 = sn * sn;
+        const double c2 = fmin(1.0, M.vortical ? fmax(M.um + M.up_m_um * sn2, 0.0) : M.sqrt_up * M.sqrt_up * sn2);
+        const double dp = r - M.rp, dm = r - M.rmn, D = dp * dm, P = r * r + a * a - a * lam;
+        const double as = sqrt(fmax(P * P - D * Q, 0.0)), s = inbound ? -as : as;
+        const double i = 1.0 / (r * D);
+        const double wp = s * wpf * dm * i, wm = s * wmf * dp * i;
+        double t;
+        if (r > 64.0 && P > 0.0) t = D * Q / (P + as) * (1.0 + 2.0 * D * i) + 2.0 * (2.0 * r - a * a) * P * i;
+        else t = (r * r + a * a) * P * (r * i) - as * (1.0 + 2.0 * D * i);
+        gt = t + a * (lam - a * (1.0 - c2)) - M.Qt * wp - M.Qtm * wm;
+        gp = a * (2.0 * r - a * lam) * (r * i) - qp * wp - qpm * wm + poln * (1.0 - M.gc * di * (1.0 - 0.5 * M.mp * cn * cn)) / (1.0 - M.qn * sn2);
+    }
+};
+
+// The anchors of a ray, kAnchorRun consecutive ones a thread (the whole warp at the same place of
+// neighbouring rays). A panel's sixteen Gauss-Legendre states come from its middle's by the addition
+// theorem, with steps that all panels of the ray share, and the middle of the next panel from this one's;
+// only the panel that holds the radial turning point (cut in two there) and the first of all, up to the
+// first sample, evaluate amplitudes at their own nodes. Bound by FP64 arithmetic: an amplitude costs some
+// seven sines and arcsines, and the kernel that took two per node spent 32.1 ms at 65536 rays x 1024 samples.
+constexpr int kAnchorRun = 2;
+
+__global__ void __launch_bounds__(kBlock) k_anchor_segments(PlanView P, Spacetime st, long long npix, double* __restrict__ anchors) {
+    const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (j >= npix) return;
+    const int nanch = int(P.get(PF_NANCH, j));
+    const int m0 = blockIdx.y * kAnchorRun, m1 = min(nanch, m0 + kAnchorRun);
+    if (m0 >= nanch) return;
+    const MarchRay<double> M = load_ray<double>(P, st, j);
+    const AnchorRates rates(M);
+    const AmScale sr(M.k), sq(M.pmu);
+    const int Man = M.Manchor;
+    const double dtau = M.dtau, fo = M.fo_d;
+    const double kr = M.c, kt = M.pscale / M.tempfac;   // arguments: c (fo - tau) and pscale (tau + offset) / tempfac
+    auto xr_at_ = [&](double tau) { return sr.state(kr * (fo - tau), M.k); };
+    auto xt_at_ = [&](double tau) { return sq.state(kt * (tau + M.poffset), M.pmu); };
+    // a panel by amplitudes at its own nodes
+    auto panel = [&](double ta, double tb, double& It, double& Ip) {
+        const double mid = 0.5 * (ta + tb), half = 0.5 * (tb - ta);
+        double s0 = 0.0, s1 = 0.0;
+        for (int i = 0; i < 16; ++i) {
+            const double tau = mid + half * c_gl_x[i];
+            double gt, gp;
+            rates.at(M, xr_at_(tau), xt_at_(tau), tau < fo, gt, gp);
+            s0 += c_gl_w[i] * gt; s1 += c_gl_w[i] * gp;
+        }
+        It += half * s0; Ip += half * s1;
+    };
+    const JS<double> x0 = xt_at_(0.0);
+    const double pc0 = polar_closed(M, 0.0, x0.sn / (M.pscale * x0.dn), x0.cn / x0.dn);
+    // the shared steps: the nodes' distances from the middle of a panel (symmetric about it), panel to panel
+    const int np = (Man + kAnchorPanelSamples - 1) / kAnchorPanelSamples;
+    const double hp = Man * dtau / np, half = 0.5 * hp;
+    JS<double> nr[8], nt[8], pr, pt;
+    if (m1 > 1) {
+        for (int i = 0; i < 8; ++i) {
+            const double d = half * fabs(c_gl_x[i]);
+            nr[i] = sr.state(kr * d, M.k); nt[i] = sq.state(kt * d, M.pmu);
+        }
+        pr = sr.state(-kr * hp, M.k); pt = sq.state(kt * hp, M.pmu);
+    }
+    for (int m = m0; m < m1; ++m) {
+        const int k = 1 + m * Man;
+        const double tau = k * dtau;
+        double* A = anchors + (M.anchor_off + m) * AF_COUNT;
+        const JS<double> xr = xr_at_(tau), xt = xt_at_(tau);
+        A[AF_XR_SN] = xr.sn; A[AF_XR_CN] = xr.cn; A[AF_XR_DN] = xr.dn;
+        A[AF_XT_SN] = xt.sn; A[AF_XT_CN] = xt.cn; A[AF_XT_DN] = xt.dn;
+        double th, cth; bool nu;
+        polar_cos(M, xt, th, cth, nu);
+        const bool reached = tau <= M.tau_valid;
+        A[AF_OK] = (reached && visible(M, cth)) ? 1.0 : 0.0;
+        A[AF_PAD] = 0.0;
+        double lead_t = 0.0, lead_p = 0.0, It = 0.0, Ip = 0.0;
+        if (reached) {
+            // closed-form parts at tau, accumulated from the observer
+            const double r = radius(M, xr);
+            const double F = r + 2.0 * log(r);
+            const double L = (M.scattering && tau > fo) ? F - 2.0 * (M.r4 + 2.0 * log(M.r4)) : -F;
+            const double lp = log((r - st.rp) / r) / M.sp, lm = log((r - st.rmn) / r) / M.sm;
+            lead_t = L + M.Qt * lp + M.Qtm * lm;
+            lead_p = M.Qphi * lp + M.Qphim * lm + polar_closed(M, tau, xt.sn / (M.pscale * xt.dn), xt.cn / xt.dn) - pc0;
+            // smooth part over (previous anchor, tau]
+            if (m == 0) {
+                panel(0.0, (M.scattering && fo < tau) ? fo : tau, It, Ip);
+                if (M.scattering && fo < tau) panel(fo, tau, It, Ip);
+            } else {
+                const double ta = (1 + (m - 1) * Man) * dtau;
+                JS<double> yr = xr_at_(ta + half), yt = xt_at_(ta + half);
+                int split = -1;
+                for (int q = 0; q < np; ++q) {
+                    if (q > 0) { yr = jadd(yr, pr, M.k); yt = jadd(yt, pt, M.pmu); }
+                    const double a0 = ta + q * hp, mid = a0 + half;
+                    if (M.scattering && a0 < fo && fo < a0 + hp) { split = q; continue; }   // after the loop: the warp stays together
+                    const bool inbound = mid < fo;
+                    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 1
+                    for (int i = 0; i < 8; ++i) {
+                        // tau = mid -+ d: the radial argument runs backwards
+                        const JS<double> dr = nr[i], dt = nt[i], er = {-dr.sn, dr.cn, dr.dn}, et = {-dt.sn, dt.cn, dt.dn};
+                        double g0, p0, g1, p1;
+                        rates.at(M, jadd(yr, dr, M.k), jadd(yt, et, M.pmu), inbound, g0, p0);
+                        rates.at(M, jadd(yr, er, M.k), jadd(yt, dt, M.pmu), inbound, g1, p1);
+                        s0 += c_gl_w[i] * (g0 + g1); s1 += c_gl_w[i] * (p0 + p1);
+                    }
+                    It += half * s0; Ip += half * s1;
+                }
+                if (split >= 0) {
+                    panel(ta + split * hp, fo, It, Ip);
+                    panel(fo, split == np - 1 ? tau : ta + (split + 1) * hp, It, Ip);
+                }
+            }
+        }
+        A[AF_T] = lead_t; A[AF_PHI] = lead_p;
+        A[AF_SEG_T] = It; A[AF_SEG_PHI] = Ip;
+    }
 }
 
 __global__ void k_anchor_prefix(long long npix, long long npad, const double* __restrict__ f, const long long* __restrict__ aoff,
@@ -351,13 +453,17 @@ __global__ void k_splat_table(SetDesc d, double* __restrict__ tab) {
 // ---- kernels: the fused march with its consumers -----------------------------------------------------
 
 template <class T>
-__device__ __forceinline__ void ks_coords(T a, T r, T th, T ph, T& x, T& y, T& z, T& sth, T& cth) {
+__device__ __forceinline__ void ks_position(T a, T r, T sth, T cth, T ph, T& x, T& y, T& z) {
     T temp = sqrt(T(1) - a * a);
     T rp = T(1) + temp, rm = T(1) - temp;
     T phks = ph + a / (T(2) * temp) * log(fabs((r - rp + keps<T>()) / (r - rm + keps<T>()))) - atan2(a, r);
-    sth = sin(th); cth = cos(th);
     T sp = sin(phks), cp = cos(phks);
     x = r * sth * cp; y = r * sth * sp; z = r * cth;
+}
+template <class T>
+__device__ __forceinline__ void ks_coords(T a, T r, T th, T ph, T& x, T& y, T& z, T& sth, T& cth) {
+    sth = sin(th); cth = cos(th);
+    ks_position(a, r, sth, cth, ph, x, y, z);
 }
 
 }  // namespace
@@ -394,8 +500,10 @@ struct ThinSink {
     T eta, lam;
     __device__ void operator()(int, const Sample<T>& s) {
         if (!(s.ok && rh_lo < s.r && s.r < T(1e3))) return;
-        T x, y, z, sth, cth;
-        ks_coords(a, s.r, s.theta, s.phi, x, y, z, sth, cth);
+        // sin theta from cos theta: the march's angle would be one acos, sin and cos more per sample
+        const T cth = s.cos_theta, sth = sqrt(fmax((T(1) - cth) * (T(1) + cth), T(0)));
+        T x, y, z;
+        ks_position(a, s.r, sth, cth, s.phi, x, y, z);
         T t = t_obs - s.t;
         T jt = T(0);
         for (int i = 0; i < nsplat; ++i) {
@@ -411,22 +519,47 @@ struct ThinSink {
     }
 };
 
+// The thin image: a ray is marched in nseg pieces (a power of two), one thread each, the threads of a
+// piece side by side, so that a warp's threads are neighbouring rays at the same depth; the pieces' sums (and anchor residuals) meet in shared memory in depth order. Bound by the
+// latency of the FP64 march (every sample is a chain of logarithms, arctangents and divisions): one
+// thread per ray kept 4 warps per SM at 128 x 128 rays.
 template <class T>
-__global__ void k_thin(PlanView P, Spacetime st, long long npix, const double* __restrict__ tab64, int nsplat, double t_obs,
+__global__ void k_thin(PlanView P, Spacetime st, long long npix, const double* __restrict__ tab64, int nsplat, double t_obs, int nseg,
                        const long long* __restrict__ perm, double* __restrict__ out, double* __restrict__ resid_t,
                        double* __restrict__ resid_phi) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double part[3][kBlock];
     T* tab = reinterpret_cast<T*>(smem);
     for (int q = threadIdx.x; q < nsplat * ST_COUNT; q += blockDim.x) tab[q] = T(tab64[q]);
     __syncthreads();
-    long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (j >= npix) return;
-    MarchRay<T> R = load_ray<T>(P, st, j);
-    ThinSink<T> sink{tab, nsplat, T(t_obs), T(st.a), T(st.rh * (1 + 1e-3)), T(R.dtau), T(0), R.eta, R.lam};
-    double rt, rp;
-    march(P, st, j, R, sink, rt, rp);
-    out[perm ? perm[j] : j] = double(sink.acc);   // sorted order, or screen order through the permutation
+    const int nr = kBlock / nseg, seg = threadIdx.x / nr;
+    const long long j = blockIdx.x * (long long)nr + threadIdx.x % nr;
+    double rt = 0.0, rp = 0.0, acc = 0.0;
+    if (j < npix) {
+        MarchRay<T> R = load_ray<T>(P, st, j);
+        ThinSink<T> sink{tab, nsplat, T(t_obs), T(st.a), T(st.rh * (1 + 1e-3)), T(R.dtau), T(0), R.eta, R.lam};
+        // pieces of whole re-anchoring intervals: each starts from the anchor table
+        const int len = ((R.nsamp + nseg - 1) / nseg + st.M - 1) / st.M * st.M;
+        march_part(P, j, R, sink, 1 + seg * len, 1 + (seg + 1) * len, rt, rp);
+        acc = double(sink.acc);
+    }
+    part[0][threadIdx.x] = acc; part[1][threadIdx.x] = rt; part[2][threadIdx.x] = rp;
+    __syncthreads();
+    if (seg > 0 || j >= npix) return;
+    for (int s = 1; s < nseg; ++s) {
+        acc += part[0][threadIdx.x + s * nr];
+        rt = fmax(rt, part[1][threadIdx.x + s * nr]);
+        rp = fmax(rp, part[2][threadIdx.x + s * nr]);
+    }
+    out[perm ? perm[j] : j] = acc;   // sorted order, or screen order through the permutation
     if (resid_t) { resid_t[j] = rt; resid_phi[j] = rp; }
+}
+
+// Pieces per ray: one for each re-anchoring interval, up to 16 (a power of two).
+int thin_pieces(const Spacetime& st) {
+    int nseg = 1;
+    while (nseg < 16 && 2 * nseg * (long long)st.M <= st.N) nseg *= 2;
+    return nseg;
 }
 
 // The allocation-free thin-image variant (ks_thin_image_noalloc) keeps its splat table in this
@@ -1462,9 +1595,8 @@ int regenerate_impl(ks_context* c, double a, double theta_o, int32_t nsamples, i
     c->ranges[2] = cnt[0]; c->ranges[3] = cnt[0] + cnt[1];
     c->ranges[4] = cnt[0] + cnt[1]; c->ranges[5] = n;
     KS_CUDA(c, c->anchors.ensure(size_t(c->total_anchors) * AF_COUNT * sizeof(double)));
-    dim3 grid(nblocks(n), c->max_nanch);
-    k_anchor_segments<<<grid, kBlock, 0, c->stream>>>(st, c->alpha.as<double>(), c->beta.as<double>(), c->perm.as<long long>(), n, npad,
-                                                       c->plan.as<double>(), c->aoff.as<long long>(), c->anchors.as<double>());
+    dim3 grid(nblocks(n), (c->max_nanch + kAnchorRun - 1) / kAnchorRun);
+    k_anchor_segments<<<grid, kBlock, 0, c->stream>>>(plan_view(c), st, n, c->anchors.as<double>());
     c->launches++;
     KS_CUDA(c, cudaGetLastError());
     k_anchor_prefix<<<nblocks(n), kBlock, 0, c->stream>>>(n, npad, c->plan.as<double>(), c->aoff.as<long long>(), c->anchors.as<double>());
@@ -1572,14 +1704,15 @@ int ks_thin_image(ks_context* c, const double* params, int32_t nsplat, double t_
     KS_CUDA(c, c->out_sorted.ensure(n * sizeof(double)));
     size_t smem = size_t(nsplat) * ST_COUNT * (precision == KS_FP64 ? sizeof(double) : sizeof(float));
     if (smem > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", nsplat);
+    const int nseg = thin_pieces(c->st);
     cudaEventRecord(c->ev0, c->stream);
     if (precision == KS_FP64) {
         KS_CUDA(c, cudaFuncSetAttribute(k_thin<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<double><<<nblocks(n), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nullptr,
+        k_thin<double><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nseg, nullptr,
                                                                  c->out_sorted.as<double>(), c->resid_t.as<double>(), c->resid_phi.as<double>());
     } else {
         KS_CUDA(c, cudaFuncSetAttribute(k_thin<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<float><<<nblocks(n), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nullptr,
+        k_thin<float><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nseg, nullptr,
                                                                 c->out_sorted.as<double>(), nullptr, nullptr);
     }
     cudaEventRecord(c->ev1, c->stream);
@@ -2997,12 +3130,13 @@ int ks_thin_image_noalloc(ks_context* c, const double* params, int32_t nsplat, d
     }
     const long long* perm = order == KS_ORDER_SCREEN ? c->perm.as<long long>() : nullptr;
     const size_t smem = size_t(nsplat) * ST_COUNT * (precision == KS_FP64 ? sizeof(double) : sizeof(float));
+    const int nseg = thin_pieces(c->st);
     if (precision == KS_FP64) {
         KS_CUDA(c, cudaFuncSetAttribute(k_thin<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<double><<<nblocks(n), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, perm, out, nullptr, nullptr);
+        k_thin<double><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, nseg, perm, out, nullptr, nullptr);
     } else {
         KS_CUDA(c, cudaFuncSetAttribute(k_thin<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<float><<<nblocks(n), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, perm, out, nullptr, nullptr);
+        k_thin<float><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, nseg, perm, out, nullptr, nullptr);
     }
     c->launches++;
     KS_CUDA(c, cudaGetLastError());

@@ -261,13 +261,16 @@ __device__ __forceinline__ JS<T> load_js(const double* rec, int off) {
 // march starts at the last anchor at or before k_begin (its Jacobi states, t~ and phi from the table)
 // and runs silently up to k_begin, so the lanes of a warp call f the same number of times whatever
 // their anchor spacing. At every anchor the quadrature's t~ and phi are replaced by the anchor's; with
-// RESID the largest |quadrature - anchor| of the ray (cache.residual_t / residual_phi) is tracked.
+// RESID the largest |quadrature - anchor| of the range's intervals (cache.residual_t / residual_phi) is
+// tracked: a range that ends in front of an anchor marches silently onto it, so that the ranges of a ray
+// between them check every anchor.
 template <bool RESID, class T, class F>
 __device__ __forceinline__ void march_impl(const PlanView& P, long long j, const MarchRay<T>& R, F& f, int k_begin, int k_end,
                                            double& resid_t, double& resid_phi) {
     double rt = 0.0, rphi = 0.0;
     if (k_end > R.nsamp + 1) k_end = R.nsamp + 1;
     if (k_begin < k_end) {
+        const int k_stop = k_end + ((RESID && k_end <= R.nsamp && (k_end - 1) % R.Manchor == 0) ? 1 : 0);
         const double dtau = R.dtau;
         const double h = dtau / 2.0;
         int m = (k_begin - 1) / R.Manchor;
@@ -286,7 +289,7 @@ __device__ __forceinline__ void march_impl(const PlanView& P, long long j, const
         }
         int next_anchor = ka + R.Manchor;
         ++m;
-        for (int k = ka + 1; k < k_end; ++k) {
+        for (int k = ka + 1; k < k_stop; ++k) {
             double ta = (k - 1) * dtau, tb = k * dtau;
             xr = jstep(xr, R.dr, R.k);
             xt = jstep(xt, R.dth, R.pmu);
@@ -335,7 +338,7 @@ __device__ __forceinline__ void march_impl(const PlanView& P, long long j, const
                 ++m;
                 next_anchor += R.Manchor;
             }
-            if (k >= k_begin) {
+            if (k >= k_begin && (!RESID || k < k_end)) {
                 Sample<T> s{T(t), pb.r, pb.theta, pb.cth, T(phi), pb.nur, pb.nuth, (tb <= R.tau_valid) && visible(R, pb.cthp)};
                 f(k, s);
             }
@@ -353,6 +356,13 @@ __device__ __forceinline__ void march(const PlanView& P, const Spacetime& st, lo
                                       F& f, double& resid_t, double& resid_phi) {
     (void)st;
     march_impl<true>(P, j, R, f, 1, R.nsamp + 1, resid_t, resid_phi);
+}
+
+// March samples [k_begin, k_end) of ray j with the anchor residuals of their intervals.
+template <class T, class F>
+__device__ __forceinline__ void march_part(const PlanView& P, long long j, const MarchRay<T>& R, F& f, int k_begin, int k_end,
+                                           double& resid_t, double& resid_phi) {
+    march_impl<true>(P, j, R, f, k_begin, k_end, resid_t, resid_phi);
 }
 
 // March samples [k_begin, k_end) of ray j (no residuals): the work segments of the sample stream.

@@ -69,6 +69,7 @@ __device__ __forceinline__ float freduce(float x) {
 }
 __device__ __forceinline__ void fsincos(float x, float& s, float& c) { __sincosf(freduce(x), &s, &c); }
 __device__ __forceinline__ float fcos(float x) { return __cosf(freduce(x)); }
+__device__ __forceinline__ void fsincos(double x, double& s, double& c) { sincos(x, &s, &c); }
 template <class T> __device__ __forceinline__ void fsincos(const T& x, T& s, T& c) { s = sin(x); c = cos(x); }
 template <class T> __device__ __forceinline__ T fcos(const T& x) { return cos(x); }
 // FP32 duals: the value by the reduced hardware pair, the partials by the chain rule
