@@ -36,7 +36,7 @@ UNIT = "ray-samples/s"
 FLOPS = {"samples": 330, "valid_samples": 95, "splat_tests": 22, "weights": 32, "coefficients": 170,
          "frames": 115, "steps": 1150}
 SFU = {"samples": 12, "valid_samples": 9, "splat_tests": 2, "weights": 1, "coefficients": 22, "frames": 4, "steps": 12}
-# k_consume's DRAM traffic per ray-sample: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch
+# k_transport's DRAM traffic per ray-sample: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch
 # of this workload at full size (256x256, N = 1024, 3 frequencies: 2.1709e9 + 0.1235e9 B over 65536 x 1024
 # ray-samples; reads = the FP32 sample stream, 32 B per ray-sample, partly still in L2 after k_stream
 # writes it, + the plan; writes = segment states)
@@ -214,18 +214,18 @@ def run_ours(args):
     e2e_ms = max_over_ranks(e2e_ms, dev)
     e2e_value = units_per_step * world / (e2e_ms / 1e3)
 
-    # roofline of the dominant kernel: k_consume on the mixed path (the march runs before it in
-    # k_stream, so its per-sample flops are left out), k_polarized<double> on the FP64 plain path;
+    # roofline of the dominant kernel: k_transport on the mixed path (the march runs before it in
+    # k_stream, so its per-sample flops are left out), k_transport<double> on the FP64 plain path;
     # algorithmic FP32 (FP64) work per launch / its CUDA-event time
     if prec != ks.KS_FP64 and consume_launches > 0:
-        kname = "k_consume"
+        kname = "k_transport"
         flops = sum(FLOPS[k] * counts[k] for k in FLOPS if k != "samples")
         sfu = sum(SFU[k] * counts[k] for k in SFU if k != "samples")
         launch_ms = consume_ms / consume_launches
         launches_per_step = consume_launches / args.steps
         traffic = CONSUME_TRAFFIC_PER_RAY_SAMPLE * cache.npix * c["N"]
     else:
-        kname = "k_polarized<double,1>"
+        kname = "k_transport<double>"
         flops = sum(FLOPS[k] * counts[k] for k in FLOPS)
         sfu = sum(SFU[k] * counts[k] for k in SFU)
         launch_ms = render_ms / max(render_launches, 1)
@@ -246,7 +246,7 @@ def run_ours(args):
                    "l2": "no flush: the per-ray FP64 plan + anchor table (~150 MB) exceeds the 126 MB L2"},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
-                     "traffic": traffic, "traffic_source": "ncu DRAM bytes of one k_consume launch of this workload (256x256, N=1024, 3 frequencies)"
+                     "traffic": traffic, "traffic_source": "ncu DRAM bytes of one k_transport launch of this workload (256x256, N=1024, 3 frequencies)"
                      if traffic else None,
                      "peak_source": "nominal FP32 pipe (148 SMs x 128 lanes x 2 x max SM clock); MEASURED_PEAKS.json has no FP32 figure",
                      "kernel": kname, "kernel_ms": launch_ms, "flops_per_launch": flops_per_launch,

@@ -291,7 +291,7 @@ int ks_graph_destroy(ks_context* ctx);
  * the hook off to render again. */
 int ks_set_stage_test(ks_context* ctx, int32_t on);
 
-/* Device time (CUDA events on the context stream) of the persistent consumer k_consume alone in the
+/* Device time (CUDA events on the context stream) of the persistent consumer k_transport alone in the
  * mixed ks_render calls since the last reset, and its launch count (one per mixed render). */
 int ks_consume_stats(ks_context* ctx, double* consume_ms, long long* launches, int reset);
 

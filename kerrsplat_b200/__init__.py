@@ -241,7 +241,7 @@ class GeodesicCache:
         return ms.value, n.value, fl.value
 
     def consume_stats(self, reset=False):
-        """(ms, launches) of k_consume alone in the mixed renders since the last reset."""
+        """(ms, launches) of k_transport alone in the mixed renders since the last reset."""
         ms = ctypes.c_double()
         n = ctypes.c_longlong()
         self._check(self._lib.ks_consume_stats(self._ctx, ctypes.byref(ms), ctypes.byref(n), int(reset)))

@@ -7,7 +7,7 @@
 //     exclusive scan of anchor counts -> k_anchor_segments (one thread per (ray, anchor): Jacobi
 //     states, validity, closed-form parts and the Gauss-Legendre integral of the smooth part since
 //     the previous anchor) -> k_anchor_prefix (per-ray running sums).
-//   ks_thin_image / ks_render: k_splat_table (per-splat FP64 constants) -> k_thin / k_polarized
+//   ks_thin_image / ks_render: k_splat_table (per-splat FP64 constants) -> k_thin / k_transport
 //     (one thread per ray, the fused march with the consumer folded over the samples) -> k_unsort.
 #include <cub/cub.cuh>
 #include <cudaTypedefs.h>
@@ -27,11 +27,11 @@
 
 using namespace ks;
 
-__constant__ MomentCoeffs c_moments;
+static __constant__ MomentCoeffs c_moments;
+
+#include "ks_context.cuh"
 
 namespace {
-
-constexpr int kBlock = 128;
 
 // ---- kernels: regenerate ---------------------------------------------------------------------------
 
@@ -452,23 +452,7 @@ __global__ void k_splat_table(SetDesc d, double* __restrict__ tab) {
 
 // ---- kernels: the fused march with its consumers -----------------------------------------------------
 
-template <class T>
-__device__ __forceinline__ void ks_position(T a, T r, T sth, T cth, T ph, T& x, T& y, T& z) {
-    T temp = sqrt(T(1) - a * a);
-    T rp = T(1) + temp, rm = T(1) - temp;
-    T phks = ph + a / (T(2) * temp) * log(fabs((r - rp + keps<T>()) / (r - rm + keps<T>()))) - atan2(a, r);
-    T sp = sin(phks), cp = cos(phks);
-    x = r * sth * cp; y = r * sth * sp; z = r * cth;
-}
-template <class T>
-__device__ __forceinline__ void ks_coords(T a, T r, T th, T ph, T& x, T& y, T& z, T& sth, T& cth) {
-    sth = sin(th); cth = cos(th);
-    ks_position(a, r, sth, cth, ph, x, y, z);
-}
-
 }  // namespace
-
-#include "ks_mixed.cuh"
 
 namespace {
 
@@ -569,177 +553,6 @@ int thin_pieces(const Spacetime& st) {
 // streams, two host threads) share it and race.
 constexpr int kNoAllocMaxSplats = 256;
 static __device__ __align__(256) double g_noalloc_tab[kNoAllocMaxSplats * ST_COUNT];
-
-// RadiativeTransport over a concatenated splat table (transport.jl:171-198, polarized.jl:121-150,
-// populations.jl:70-104), CH (t_obs, nu) combinations per thread sharing the march.
-template <class T, int CH>
-struct PolSink {
-    const T* tab; int ntot;
-    const T* knots;   // the knot array of knot splats (after the table)
-    T t_obs[CH], nu[CH], nuh[CH], Lnu[CH];
-    int nc;
-    T a, rh_lo, dtau, alpha, beta, eta, lam, a_sin_tho, slab;
-    int nmax;
-    T P[CH][16], S[CH][4];
-    T zprev; int wn; bool inside, crossed, zset;
-    // event counts of this thread (the algorithmic-work model of the roofline): samples, valid
-    // samples, splat tests, weights evaluated, coefficient evaluations, frames, steps
-    unsigned int ev[7];
-
-    __device__ void init() {
-        for (int q = 0; q < 7; ++q) ev[q] = 0;
-        for (int c = 0; c < CH; ++c) {
-            for (int q = 0; q < 16; ++q) P[c][q] = (q % 5 == 0) ? T(1) : T(0);
-            for (int q = 0; q < 4; ++q) S[c][q] = T(0);
-        }
-        wn = 0; inside = false; crossed = false; zset = false; zprev = T(0);
-    }
-
-    __device__ void wind(T z) {   // step.jl:379-398
-        if (!zset) { zprev = z; zset = true; inside = fabs(z) < slab; crossed = false; return; }
-        bool inside_now = fabs(z) < slab;
-        bool crossing = zprev * z < T(0);
-        if (inside || inside_now) {
-            crossed = crossed || crossing;
-            if (inside && !inside_now) { if (crossed) wn += 1; crossed = false; }
-            else if (!inside && inside_now) { crossed = crossing; }
-            inside = inside_now;
-        } else if (crossing) {
-            wn += 1;
-        }
-        zprev = z;
-    }
-
-    __device__ void operator()(int, const Sample<T>& s) {
-        ev[0]++;
-        if (!(s.ok && s.r > rh_lo)) return;
-        ev[1]++;
-        if (nmax >= 0) {
-            wind(s.r * cos(s.theta));
-            if (wn > nmax) return;
-        }
-        T x, y, z, sth, cth;
-        ks_coords(a, s.r, s.theta, s.phi, x, y, z, sth, cth);
-        T j4[CH][4], a4[CH][4], r3[CH][3];
-        bool active[CH];
-        for (int c = 0; c < CH; ++c) {
-            active[c] = false;
-            for (int q = 0; q < 4; ++q) { j4[c][q] = T(0); a4[c][q] = T(0); }
-            for (int q = 0; q < 3; ++q) r3[c][q] = T(0);
-        }
-        bool have_frame = false;
-        SampleFrame<T> F;
-        for (int i = 0; i < ntot; ++i) {
-            const T* p = tab + i * ST_COUNT;
-            const int kind = int(p[ST_KIND]);
-            bool fr_done = false;
-            LFrame<T> lf;
-            for (int c = 0; c < CH; ++c) {
-                if (c >= nc) break;
-                T t = t_obs[c] - s.t;
-                T q;
-                ev[2]++;
-                if (!any_exponent(p, knots, t, x, y, z, q)) continue;
-                ev[3]++;
-                T G = exp(-q);
-                if (!(G > T(kWEIGHT_CUTOFF))) continue;
-                if (!have_frame) { F = sample_frame(a, s.r, s.theta, sth, cth, eta, lam, s.nur, s.nutheta); have_frame = true; }
-                ev[4]++;
-                if (!fr_done) {
-                    ev[5]++;
-                    lf = local_frame(F, p[ST_U1], p[ST_U2], p[ST_U3], p[ST_BHX], p[ST_BHY], p[ST_BHZ], p[ST_BZERO] != T(0),
-                                     alpha, beta, a_sin_tho);
-                    fr_done = true;
-                }
-                T nuf = nu[c] / lf.g;
-                T thb = acos(fmin(T(1), fmax(T(-1), lf.cosB)));
-                T ne = p[ST_NE] * G;
-                Coef<T> cf;
-                if (kind == KS_POWERLAW22)
-                    cf = powerlaw(ne, p[ST_P], p[ST_GMIN], p[ST_GSPAN], p[ST_GAMJ], p[ST_GAMA], p[ST_BMAG], nuf, thb);
-                else if (kind == KS_KAPPA22)
-                    cf = kappa(ne, p[ST_KAP], p[ST_W], p[ST_HYP], p[ST_G43], p[ST_G2], p[ST_GQ], p[ST_GP], p[ST_GK2], p[ST_KB], p[ST_BMAG], nuf, thb);
-                else
-                    cf = thermal(ne, p[ST_TE], p[ST_F0], p[ST_KR], p[ST_BMAG], nuf, thb);
-                // screen_coefficients (transport.jl:265-270): cap, invariants at nu/g, rotate by 2 chi
-                if (!(cf.jI > T(0) || cf.aI > T(0) || cf.rQ != T(0) || cf.rV != T(0))) continue;
-                T fe = cap_factor(cf.jI, cf.jQ, cf.jV, T(0.99));
-                T fa = cap_factor(cf.aI, cf.aQ, cf.aV, T(0.99));
-                T nh = nuf / T(kNU0);
-                T i2 = T(1) / (nh * nh);
-                T s2c = lf.s2c, c2c = lf.c2c;
-                T jQ = cf.jQ * fe * i2, aQ = cf.aQ * fa * nh, rQ = cf.rQ * nh;
-                j4[c][0] += cf.jI * i2; j4[c][1] += jQ * c2c; j4[c][2] += jQ * s2c; j4[c][3] += cf.jV * fe * i2;
-                a4[c][0] += nh * cf.aI; a4[c][1] += aQ * c2c; a4[c][2] += aQ * s2c; a4[c][3] += cf.aV * fa * nh;
-                r3[c][0] += rQ * c2c; r3[c][1] += rQ * s2c; r3[c][2] += nh * cf.rV;
-                active[c] = true;
-            }
-        }
-        T Sg = s.r * s.r + a * a * cos(s.theta) * cos(s.theta);
-        for (int c = 0; c < CH; ++c) {
-            if (c >= nc || !active[c]) continue;
-            T Dl = Lnu[c] * Sg * dtau;
-            ev[6]++;
-            T O[16], E[4];
-            transfer_step(c_moments, j4[c], a4[c], r3[c], Dl, O, E);
-            // advance (step.jl:347): S += P E, P = P O
-            T Pn[16];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                S[c][r] += P[c][4 * r] * E[0] + P[c][4 * r + 1] * E[1] + P[c][4 * r + 2] * E[2] + P[c][4 * r + 3] * E[3];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    Pn[4 * r + q] = P[c][4 * r] * O[q] + P[c][4 * r + 1] * O[4 + q] + P[c][4 * r + 2] * O[8 + q] + P[c][4 * r + 3] * O[12 + q];
-            }
-#pragma unroll
-            for (int q = 0; q < 16; ++q) P[c][q] = Pn[q];
-        }
-    }
-};
-
-template <class T, int CH>
-__global__ void __launch_bounds__(kBlock) k_polarized(PlanView P, Spacetime st, long long npix, const double* __restrict__ tab64, int ntot,
-                                                      const double* __restrict__ ct, const double* __restrict__ cnu, int ncombo, double L,
-                                                      int nmax, double slab, double* __restrict__ out, double* __restrict__ resid_t,
-                                                      double* __restrict__ resid_phi, unsigned long long* __restrict__ counters, int nkv) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    T* tab = reinterpret_cast<T*>(smem);
-    for (int q = threadIdx.x; q < ntot * ST_COUNT + nkv; q += blockDim.x) tab[q] = T(tab64[q]);
-    __syncthreads();
-    long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (j >= npix) return;
-    const int c0 = blockIdx.y * CH;
-    MarchRay<T> R = load_ray<T>(P, st, j);
-    PolSink<T, CH> sink;
-    sink.tab = tab; sink.ntot = ntot; sink.knots = tab + ntot * ST_COUNT;
-    sink.nc = min(CH, ncombo - c0);
-    for (int c = 0; c < CH; ++c) {
-        int cc = min(c0 + c, ncombo - 1);
-        sink.t_obs[c] = T(ct[cc]); sink.nu[c] = T(cnu[cc]);
-        double nh = cnu[cc] / kNU0;
-        sink.nuh[c] = T(nh);
-        sink.Lnu[c] = T(L / nh);
-    }
-    sink.a = T(st.a); sink.rh_lo = T(st.rh * (1 + 1e-3)); sink.dtau = T(R.dtau);
-    sink.alpha = T(P.get(PF_ALPHA, j)); sink.beta = T(P.get(PF_BETA, j)); sink.eta = R.eta; sink.lam = R.lam;
-    sink.a_sin_tho = T(st.a * sin(st.thetao)); sink.slab = T(slab); sink.nmax = nmax;
-    sink.init();
-    double rt, rp;
-    march(P, st, j, R, sink, rt, rp);
-    for (int c = 0; c < CH; ++c) {
-        if (c >= sink.nc) break;
-        double n3 = double(sink.nuh[c]) * double(sink.nuh[c]) * double(sink.nuh[c]);
-        double* o = out + ((long long)(c0 + c) * npix + j) * 4;
-        o[0] = double(sink.S[c][0]) * n3; o[1] = double(sink.S[c][1]) * n3;
-        o[2] = double(sink.S[c][2]) * n3; o[3] = double(sink.S[c][3]) * n3;
-    }
-    if (blockIdx.y == 0 && resid_t) { resid_t[j] = rt; resid_phi[j] = rp; }
-    if (counters) {
-        // samples are counted once per (ray, combo) as the metric counts them
-        atomicAdd(&counters[0], (unsigned long long)sink.ev[0] * sink.nc);
-        for (int q = 1; q < 7; ++q) atomicAdd(&counters[q], (unsigned long long)sink.ev[q]);
-    }
-}
 
 // ---- ipole's RIAF as a fluid model of the polarized consumer ------------------------------------
 // The reference's test/riaf_model.jl: a thick disk with power-law density and temperature, a
@@ -955,120 +768,11 @@ __global__ void k_unsort(const double* __restrict__ src, const long long* __rest
 
 // ---- the context ----------------------------------------------------------------------------------------
 
-struct DevBuf {
-    void* p = nullptr;
-    size_t n = 0;
-    DevBuf() = default;
-    DevBuf(const DevBuf&) = delete;   // one owner per allocation
-    DevBuf& operator=(const DevBuf&) = delete;
-    ~DevBuf() { release(); }
-    cudaError_t ensure(size_t bytes) {
-        if (bytes <= n) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr; n = 0;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaSuccess) n = bytes;
-        return e;
-    }
-    void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
-    template <class U> U* as() const { return reinterpret_cast<U*>(p); }
-};
-
-struct ks_context {
-    int device = 0;
-    cudaStream_t stream = nullptr;
-    std::string err;
-    long long npix = 0, npad = 0;
-    int nalpha = 0, nbeta = 0;
-    bool regenerated = false;
-    Spacetime st{};
-    DevBuf alpha, beta, key, key2, idx, perm, plan, nanch, aoff, anchors, resid_t, resid_phi, scratch;
-    DevBuf tab, combos, out_sorted, stage_in, stage_out, counters, seg_out, work, stream_buf;
-    DevBuf inv_perm, dft_tu, dft_tv, dft_a, dft_t, dft_c, dft_s, dft_in[8], dft_partial;
-    // adjoint: gradient table, stored FP64 samples (plain path), cutoffs, tails, per-ray slots,
-    // seeds, chi^2 partials; mixed path: per-sample states, activity, segment bounds, unit partials
-    DevBuf gtab, samples, kstop, tails, slots, dgrad, seeds, chi_part, chi_val, dstage;
-    DevBuf adj_state, adj_act, adj_bnd, adj_unit, adj_part, jvp_tab, jvp_in, jvp_out, st_buf;
-    DevBuf tab32;     // the splat table and knot array in FP32, padded to 16 bytes (the TMA staging source)
-    DevBuf errflag;   // set by a kernel whose bounded wait gave up
-    cudaGraph_t graph = nullptr;          // ks_render_graph_capture: one mixed render of device-resident sets
-    cudaGraphExec_t graph_exec = nullptr;
-    cudaGraph_t cgraph = nullptr;         // ks_chi2_gradient_graph_capture: one mixed chi^2 + gradient evaluation
-    cudaGraphExec_t cgraph_exec = nullptr;
-    std::vector<void*> cgraph_bufs;
-    bool capturing = false;               // inside that capture: no timing events
-    int stage_test = 0;                   // ks_set_stage_test
-    std::vector<void*> graph_bufs;        // the buffers the graph uses, as captured (a replay checks them)
-    bool samples_ready = false;
-    int tune_nt = 0, tune_units = 0;        // the autotuner's choice for the mixed forward (0: the default)
-    int nkv = 0;                            // knot values after the splat table in `tab`
-    MixedJob last_job{};                    // the segmentation of the last mixed forward pass
-    float* fwd_gstate = nullptr;            // set during the adjoint's forward pass only
-    unsigned char* fwd_gact = nullptr;
-    double adjoint_ms = 0.0;
-    long long adjoint_launches = 0;
-    bool count_events = false;
-    int tensor_path = 0;  // 3xTF32 GEMMs: 0 tcgen05 (k_gemm_tc), 1 mma.sync (k_gemm_3xtf32); ks_set_tensor_path
-    bool geo64 = false;   // mixed path: the FP64 march feeds the FP32 transport (KS_MIXED_GEO64) instead of the FP32 march
-    long long total_anchors = 0;
-    int max_nanch = 0;
-    long long ranges[6] = {0, 0, 0, 0, 0, 0};
-    // timing of the render kernels (CUDA events on the context stream)
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t evc0 = nullptr, evc1 = nullptr;   // around k_consume (the mixed path's dominant kernel)
-    cudaEvent_t evg0 = nullptr, evg1 = nullptr;   // around each 3xTF32 GEMM (outside graph captures)
-    double gemm_ms = 0.0, gemm_flops = 0.0;       // ks_gemm_stats: device time and tensor-core flops (3 x 2 M N K)
-    long long gemm_launches = 0;
-    bool consume_timed = false;
-    double consume_ms = 0.0;
-    long long consume_launches = 0;
-    double kernel_ms = 0.0;
-    long long kernel_launches = 0;
-    long long launches = 0;
-};
-
 namespace {
-
-int fail(ks_context* c, int code, const char* fmt, ...) {
-    char buf[512];
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(buf, sizeof buf, fmt, ap);
-    va_end(ap);
-    if (c) c->err = buf;
-    return code;
-}
-
-int cuda_fail(ks_context* c, cudaError_t e, const char* what) {
-    if (e == cudaErrorMemoryAllocation) return fail(c, KS_ERR_OUT_OF_MEMORY, "%s: %s", what, cudaGetErrorString(e));
-    return fail(c, KS_ERR_DEVICE, "%s: %s", what, cudaGetErrorString(e));
-}
-
-#define KS_CUDA(ctx, call)                                            \
-    do {                                                              \
-        cudaError_t e_ = (call);                                      \
-        if (e_ != cudaSuccess) return cuda_fail((ctx), e_, #call);    \
-    } while (0)
-
-bool is_device_ptr(const void* p) {
-    if (!p) return false;
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
-}
-
-// Make `src` (host or device, `bytes`) available on the device: returns the device pointer.
-int stage_in(ks_context* c, DevBuf& buf, const void* src, size_t bytes, const void** dev) {
-    if (is_device_ptr(src)) { *dev = src; return KS_OK; }
-    KS_CUDA(c, buf.ensure(bytes));
-    KS_CUDA(c, cudaMemcpyAsync(buf.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
-    *dev = buf.p;
-    return KS_OK;
-}
 
 void init_constants() {
     MomentCoeffs mc;
-    for (int n = 0; n < 10; ++n) {
+    for (int n = 0; n < 11; ++n) {
         double fact = 1.0;
         for (int m = 0; m < 24; ++m) {
             if (m > 0) fact *= m;
@@ -1077,6 +781,8 @@ void init_constants() {
         }
     }
     cudaMemcpyToSymbol(c_moments, &mc, sizeof mc);
+    forward_init(mc);
+    reverse_init(mc);
     // 16-point Gauss-Legendre nodes on [-1, 1] (Newton on P_16)
     double x[16], w[16];
     const int n = 16;
@@ -1097,14 +803,6 @@ void init_constants() {
     }
     cudaMemcpyToSymbol(c_gl_x, x, sizeof x);
     cudaMemcpyToSymbol(c_gl_w, w, sizeof w);
-}
-
-unsigned nblocks(long long n, int b = kBlock) { return unsigned((n + b - 1) / b); }
-
-PlanView plan_view(ks_context* c) {
-    PlanView P;
-    P.f = c->plan.as<double>(); P.npad = c->npad; P.anchors = c->anchors.as<double>(); P.anchor_off = c->aoff.as<long long>();
-    return P;
 }
 
 int nrows_of(int kind) {
@@ -1214,147 +912,6 @@ int check_device_flag(ks_context* c, const char* what) {
     return KS_OK;
 }
 
-// The FP32 sample stream of every ray (k_stream: the FP32 march, or the FP64 march under
-// KS_MIXED_GEO64), [k][field][npad]. Each ray is marched as up to eight segments, each starting
-// at an anchor (a multiple of M samples). At 256 x 256, N = 1024 that is 6.9 waves of 16 warps per
-// SM instead of 3.5 with four segments (the render 22.04 against 22.34 ms).
-int launch_stream(ks_context* c) {
-    const int M = c->st.M, N = c->st.N;
-    const int sseg = std::max(M, (N / 8 + M - 1) / M * M);
-    const int nsseg = (N + sseg - 1) / sseg;
-    KS_CUDA(c, c->stream_buf.ensure(size_t(N) * SM_COUNT * c->npad * sizeof(float)));
-    if (c->geo64)
-        k_stream<double><<<nblocks(c->npix * nsseg, 128), 128, 0, c->stream>>>(plan_view(c), c->st, c->npix, sseg, nsseg, c->stream_buf.as<float>());
-    else
-        k_stream<float><<<nblocks(c->npix * nsseg, 128), 128, 0, c->stream>>>(plan_view(c), c->st, c->npix, sseg, nsseg, c->stream_buf.as<float>());
-    c->launches++;
-    KS_CUDA(c, cudaGetLastError());
-    return KS_OK;
-}
-
-constexpr int kCandRun = 16;   // samples per candidate mask (16 vs the whole segment: config 5 -28%, config 2 -3%)
-
-template <int CH, int NT, int KM>
-int launch_consume(ks_context* c, const MixedJob& job0, int ntot, int nsm, int per_sm) {
-    MixedJob job = job0;
-    const int N = c->st.N;
-    constexpr int W = NT / 32;
-    const size_t smem = MixedSmem<CH>::bytes(ntot, W, c->nkv);
-    // split the sample range into segments until there are about eight work units per resident
-    // warp, so that the most expensive unit is short
-    const long long resident = (long long)nsm * per_sm * W;
-    const long long base_units = job.nchunks * job.nframes * job.nvc;
-    int nseg = 1;
-    const int units_per_warp = c->tune_units > 0 ? c->tune_units : 8;
-    while (job.nmax < 0 && base_units * nseg < units_per_warp * resident && (nseg * 2) * 16 <= N) nseg *= 2;
-    job.seg_len = (N + nseg - 1) / nseg;
-    job.nseg = (N + job.seg_len - 1) / job.seg_len;
-    job.total = base_units * job.nseg;
-    // candidate masks per run of samples (a segment's box spans the emission region in depth)
-    job.cand_len = kCandRun;
-    const double* dt = c->combos.as<double>();
-    const double* dn = dt + job.nframes;
-    job.gstate = c->fwd_gstate;
-    job.gact = c->fwd_gact;
-    c->last_job = job;
-    const size_t seg_bytes = size_t(job.nframes) * job.nfreq * job.nseg * c->npix * 20 * sizeof(float);
-    KS_CUDA(c, c->seg_out.ensure(seg_bytes));
-    KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));   // the adjoint's two counters: no move under a captured render
-    KS_CUDA(c, cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long), c->stream));
-    const long long grid = std::min<long long>(job.total / W + 1, (long long)nsm * per_sm);
-    if (!c->capturing) cudaEventRecord(c->evc0, c->stream);
-    k_consume<CH, NT, KM><<<unsigned(grid), NT, smem, c->stream>>>(
-        plan_view(c), c->st, job, c->tab32.as<float>(), ntot, dt, dn, c->stream_buf.as<float>(), c->work.as<unsigned long long>(),
-        c->seg_out.as<float>(), c->count_events ? c->counters.as<unsigned long long>() : nullptr, c->errflag.as<unsigned>());
-    if (!c->capturing) {
-        cudaEventRecord(c->evc1, c->stream);
-        c->consume_timed = true;
-    }
-    c->launches++;
-    c->kernel_launches++;
-    KS_CUDA(c, cudaGetLastError());
-    const long long nq = c->npix * (long long)job.nframes * job.nfreq;
-    k_combine<<<nblocks(nq, 256), 256, 0, c->stream>>>(job, dn, c->seg_out.as<float>(), c->out_sorted.as<double>());
-    c->launches++;
-    KS_CUDA(c, cudaGetLastError());
-    return KS_OK;
-}
-
-// Occupancy of k_consume<CH, NT, KM> with its shared memory for `ntot` splats (0 if it does not fit).
-template <int CH, int NT, int KM>
-int consume_blocks(ks_context* c, int ntot) {
-    const size_t smem = MixedSmem<CH>::bytes(ntot, NT / 32, c->nkv);
-    if (smem > 227 * 1024) return 0;
-    if (cudaFuncSetAttribute(k_consume<CH, NT, KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_consume<CH, NT, KM>, NT, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return per_sm;
-}
-
-template <int CH, int KM>
-int launch_mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab) {
-    int nsm = 0;
-    KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    // 1. the FP32 sample stream (one march per ray, shared by every frame and frequency)
-    {
-        int s = launch_stream(c);
-        if (s) return s;
-    }
-    MixedJob job;
-    job.npix = c->npix; job.npad = c->npad; job.nframes = nframes; job.nfreq = nfreq;
-    job.nvc = (nfreq + CH - 1) / CH;
-    job.nchunks = (c->npix + 31) / 32;
-    job.nmax = nmax; job.slab = float(slab); job.L = L;
-    job.nkv = c->nkv;
-    job.ch = CH;
-    job.stage_test = c->stage_test;
-    // the block size with the most resident warps (the per-warp shared memory sets the limit)
-    const int w384 = consume_blocks<CH, 384, KM>(c, ntot) * 12, w256 = consume_blocks<CH, 256, KM>(c, ntot) * 8,
-              w128 = consume_blocks<CH, 128, KM>(c, ntot) * 4;
-    const int best = std::max(w384, std::max(w256, w128));
-    if (best <= 0) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
-    // the autotuner's block size when it fits
-    if (c->tune_nt == 384 && w384 > 0) return launch_consume<CH, 384, KM>(c, job, ntot, nsm, w384 / 12);
-    if (c->tune_nt == 256 && w256 > 0) return launch_consume<CH, 256, KM>(c, job, ntot, nsm, w256 / 8);
-    if (c->tune_nt == 128 && w128 > 0) return launch_consume<CH, 128, KM>(c, job, ntot, nsm, w128 / 4);
-    if (w384 == best) return launch_consume<CH, 384, KM>(c, job, ntot, nsm, w384 / 12);
-    if (w256 == best) return launch_consume<CH, 256, KM>(c, job, ntot, nsm, w256 / 8);
-    if (w128 > 0) return launch_consume<CH, 128, KM>(c, job, ntot, nsm, w128 / 4);
-    return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
-}
-
-// The most warps of k_consume<CH, *, KM> resident per SM for an ntot-splat table.
-template <int CH, int KM>
-int resident_warps(ks_context* c, int ntot) {
-    return std::max(consume_blocks<CH, 384, KM>(c, ntot) * 12, std::max(consume_blocks<CH, 256, KM>(c, ntot) * 8,
-                                                                        consume_blocks<CH, 128, KM>(c, ntot) * 4));
-}
-
-// The frequencies of a work unit: all of them (up to four) share the march and the splat tests,
-// unless the per-thread states of four frequencies and a large splat table leave room for half as
-// many warps as two frequencies per unit would: then two (every sample is tested twice, but with the
-// block-cooperative consumer occupancy pays more: the 256-splat movie ran 4 warps per SM with four).
-template <int KM>
-int launch_mixed_km(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab) {
-    if (nfreq >= 4) {
-        if (resident_warps<2, KM>(c, ntot) >= 2 * resident_warps<4, KM>(c, ntot))
-            return launch_mixed_ch<2, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-        return launch_mixed_ch<4, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    }
-    if (nfreq == 3) return launch_mixed_ch<3, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    if (nfreq == 2) return launch_mixed_ch<2, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    return launch_mixed_ch<1, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-}
-
-int launch_mixed(ks_context* c, int ntot, const double* ht, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only) {
-    (void)ht;
-    if (ntot > 32 * kMaxSplatWords) return fail(c, KS_ERR_ARGUMENT, "the mixed path takes at most %d splats (%d)", 32 * kMaxSplatWords, ntot);
-    return thermal_only ? launch_mixed_km<1>(c, ntot, nframes, nfreq, L, nmax, slab) : launch_mixed_km<7>(c, ntot, nframes, nfreq, L, nmax, slab);
-}
-
 // Write `nvec` x npix x width doubles from the sorted device buffer to `out` (host or device) in `order`.
 int emit(ks_context* c, const double* sorted, int width, int nvec, int order, double* out) {
     size_t bytes = size_t(c->npix) * width * nvec * sizeof(double);
@@ -1431,7 +988,7 @@ int ks_context_stream(ks_context* c, void** stream) {
     return KS_OK;
 }
 
-// Accumulated device time of the render kernels (k_thin / k_polarized) since the last reset, and
+// Accumulated device time of the render kernels (k_thin / k_transport) since the last reset, and
 // the number of launches of this library's kernels.
 int ks_kernel_stats(ks_context* c, double* render_ms, long long* render_launches, long long* all_launches, int reset) {
     if (!c) return KS_ERR_ARGUMENT;
@@ -1466,7 +1023,7 @@ int ks_set_tensor_path(ks_context* c, int32_t path) {
     return KS_OK;
 }
 
-// Device time of k_consume alone in the mixed ks_render calls since the last reset, and its launches.
+// Device time of k_transport alone in the mixed ks_render calls since the last reset, and its launches.
 int ks_consume_stats(ks_context* c, double* consume_ms, long long* launches, int reset) {
     if (!c) return KS_ERR_ARGUMENT;
     if (consume_ms) *consume_ms = c->consume_ms;
@@ -1612,7 +1169,6 @@ int regenerate_impl(ks_context* c, double a, double theta_o, int32_t nsamples, i
     KS_CUDA(c, cudaMemsetAsync(c->resid_phi.p, 0, n * sizeof(double), c->stream));
     KS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->regenerated = true;
-    c->samples_ready = false;
     return KS_OK;
 }
 }  // namespace
@@ -1753,49 +1309,25 @@ int ks_render(ks_context* c, const ks_splat_set* sets, int32_t nsets, const doub
     }
     const long long n = c->npix;
     const int ncombo = nframes * nfreq;
-    std::vector<double> hc(2 * size_t(ncombo));
-    for (int fv = 0; fv < nfreq; ++fv)
-        for (int ft = 0; ft < nframes; ++ft) {
-            hc[size_t(fv) * nframes + ft] = ht[ft];
-            hc[ncombo + size_t(fv) * nframes + ft] = hnu[fv];
-        }
-    if (precision == KS_MIXED) {
-        // times then frequencies
-        hc.assign(ht.begin(), ht.end());
-        hc.insert(hc.end(), hnu.begin(), hnu.end());
-    }
+    std::vector<double> hc(ht);   // times then frequencies
+    hc.insert(hc.end(), hnu.begin(), hnu.end());
     // sized for the adjoint's layout too (times, frequencies, then per combination), so that an
     // adjoint call does not move the buffer under a captured render
     KS_CUDA(c, c->combos.ensure((size_t(nframes) + nfreq + 2 * size_t(ncombo)) * sizeof(double)));
     KS_CUDA(c, cudaMemcpyAsync(c->combos.p, hc.data(), hc.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     KS_CUDA(c, c->out_sorted.ensure(size_t(n) * 4 * ncombo * sizeof(double)));
-    const double* dct = c->combos.as<double>();
-    const double* dcn = dct + ncombo;
     if (c->count_events) {
         KS_CUDA(c, c->counters.ensure(8 * sizeof(unsigned long long)));
         KS_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
     }
     cudaEventRecord(c->ev0, c->stream);
-    if (precision == KS_FP64) {
-        // the plain path: one march per (frame, frequency), as the reference's polarized_cube does
-        size_t smem = (size_t(ntot) * ST_COUNT + c->nkv) * sizeof(double);
-        if (smem > 220 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
-        KS_CUDA(c, cudaFuncSetAttribute(k_polarized<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        for (int cc = 0; cc < ncombo; ++cc) {
-            k_polarized<double, 1><<<dim3(nblocks(n), 1), kBlock, smem, c->stream>>>(
-                plan_view(c), c->st, n, c->tab.as<double>(), ntot, dct + cc, dcn + cc, 1, L, nmax, slab,
-                c->out_sorted.as<double>() + size_t(cc) * n * 4, c->resid_t.as<double>(), c->resid_phi.as<double>(),
-                c->count_events ? c->counters.as<unsigned long long>() : nullptr, c->nkv);
-            c->launches++;
-            c->kernel_launches++;
-        }
-    } else {
-        // the mixed path: one launch over rays x (frame, frequency chunk)
-        bool thermal_only = true;
-        for (int q = 0; q < nsets; ++q) thermal_only = thermal_only && (sets[q].kind == KS_THERMAL21 || sets[q].nsplat == 0);
-        int s = launch_mixed(c, ntot, ht.data(), nframes, nfreq, L, nmax, slab, thermal_only);
-        if (s) return s;
-    }
+    bool thermal_only = true;
+    for (int q = 0; q < nsets; ++q) thermal_only = thermal_only && (sets[q].kind == KS_THERMAL21 || sets[q].nsplat == 0);
+    if (precision == KS_FP64 && (size_t(ntot) * ST_COUNT + c->nkv) * sizeof(double) > 220 * 1024)
+        return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
+    int sl = precision == KS_FP64 ? launch_plain(c, ntot, nframes, nfreq, L, nmax, slab, thermal_only)
+                                  : launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, thermal_only);
+    if (sl) return sl;
     cudaEventRecord(c->ev1, c->stream);
     KS_CUDA(c, cudaGetLastError());
     int s = emit(c, c->out_sorted.as<double>(), 4, ncombo, order, out);
@@ -1811,8 +1343,7 @@ int ks_render(ks_context* c, const ks_splat_set* sets, int32_t nsets, const doub
         c->consume_launches++;
         c->consume_timed = false;
     }
-    if (precision != KS_FP64) return check_device_flag(c, "ks_render");
-    return KS_OK;
+    return check_device_flag(c, "ks_render");
 }
 
 int ks_riaf_image(ks_context* c, const double* model, int32_t pandya, const double* nus, int32_t nfreq, double L, int32_t precision,
@@ -1862,7 +1393,7 @@ int ks_riaf_image(ks_context* c, const double* model, int32_t pandya, const doub
 
 // The device buffers a captured render reads or writes (a replay requires them unmoved).
 std::vector<void*> graph_buffers(const ks_context* c) {
-    return {c->tab.p, c->tab32.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->combos.p, c->errflag.p,
+    return {c->tab.p, c->tab32.p, c->rows.p, c->kstop.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->combos.p, c->errflag.p,
             c->perm.p, c->plan.p, c->anchors.p, c->aoff.p};
 }
 
@@ -1939,7 +1470,7 @@ int ks_render_graph_capture(ks_context* c, const ks_splat_set* sets, int32_t nse
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
     status = capture_tables(c, sets, nsets, ntot, false);
-    if (status == KS_OK) status = launch_mixed(c, ntot, nullptr, nframes, nfreq, L, nmax, slab, thermal_only);
+    if (status == KS_OK) status = launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, thermal_only);
     if (status == KS_OK) status = emit(c, c->out_sorted.as<double>(), 4, nframes * nfreq, order, out);
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(c->stream, &g);
@@ -2013,25 +1544,6 @@ __global__ void k_accumulate(double* __restrict__ dst, const double* __restrict_
     if (q < n) dst[q] = (accumulate ? dst[q] : 0.0) + src[q];
 }
 
-// The stored FP64 samples of every ray (the reference's store_samples cache, built once per regenerate).
-int ensure_samples(ks_context* c, StoredSamples* S) {
-    const long long n = c->npix;
-    const size_t ns = size_t(n) * c->st.N;
-    KS_CUDA(c, c->samples.ensure(ns * (4 * sizeof(double) + 1)));
-    double* d = c->samples.as<double>();
-    unsigned char* fl = reinterpret_cast<unsigned char*>(d + 4 * ns);
-    if (!c->samples_ready) {
-        KS_CUDA(c, cudaMemsetAsync(fl, 0, ns, c->stream));   // samples past a ray's count stay invalid
-        k_march_store<<<nblocks(n), kBlock, 0, c->stream>>>(plan_view(c), c->st, n, d, d + ns, d + 2 * ns, d + 3 * ns, fl,
-                                                              c->resid_t.as<double>(), c->resid_phi.as<double>());
-        c->launches++;
-        KS_CUDA(c, cudaGetLastError());
-        c->samples_ready = true;
-    }
-    *S = StoredSamples{d, d + ns, d + 2 * ns, d + 3 * ns, fl};
-    return KS_OK;
-}
-
 // Stage `count` elements of `src` (host or device) into `buf`; returns the device pointer.
 template <class U>
 int stage_dev(ks_context* c, DevBuf& buf, const U* src, size_t count, const U** dev) {
@@ -2040,96 +1552,6 @@ int stage_dev(ks_context* c, DevBuf& buf, const U* src, size_t count, const U** 
     int s = stage_in(c, buf, src, count * sizeof(U), &d);
     *dev = reinterpret_cast<const U*>(d);
     return s;
-}
-
-// Occupancy of k_adj_elements<CH, NT> with its shared memory for `ntot` splats (0 if it does not fit).
-template <int CH, int NT>
-int adjoint_blocks(ks_context* c, int ntot, bool global_acc) {
-    const size_t smem = AdjSmem<CH>::bytes(ntot, NT / 32, global_acc);
-    if (smem > 227 * 1024) return 0;
-    if (cudaFuncSetAttribute(k_adj_elements<CH, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_elements<CH, NT>, NT, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
-    return per_sm;
-}
-
-template <int CH, int NT>
-int launch_adjoint_mixed_nt(ks_context* c, int ntot, int per_sm, const double* dt, const double* dn, bool global_acc) {
-    int nsm = 0;
-    KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    const MixedJob& job = c->last_job;
-    const long long ncombo = (long long)job.nframes * job.nfreq;
-    KS_CUDA(c, c->adj_bnd.ensure(size_t(ncombo) * job.nseg * 8 * c->npix * sizeof(float)));
-    k_adj_bounds<<<nblocks(c->npix * ncombo, 256), 256, 0, c->stream>>>(job, dn, c->seg_out.as<float>(), c->seeds.as<double>(),
-                                                                        c->adj_bnd.as<float>());
-    c->launches++;
-    KS_CUDA(c, cudaGetLastError());
-    const long long gsz = (long long)ntot * GR_COUNT;
-    KS_CUDA(c, c->adj_unit.ensure(size_t(job.total) * gsz * sizeof(float)));
-    KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));
-    KS_CUDA(c, cudaMemsetAsync(c->work.p, 0, 2 * sizeof(unsigned long long), c->stream));
-    // the step phase
-    {
-        constexpr int NS = 256, WS = NS / 32;
-        const size_t smem = AdjSmem<CH>::step_bytes(WS);
-        KS_CUDA(c, cudaFuncSetAttribute(k_adj_steps<CH, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per = 0;
-        KS_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_adj_steps<CH, NS>, NS, smem));
-        const long long grid = std::min<long long>(job.total / WS + 1, (long long)nsm * std::max(per, 1));
-        k_adj_steps<CH, NS><<<unsigned(grid), NS, smem, c->stream>>>(c->st, job, dn, c->plan.as<double>(), c->stream_buf.as<float>(),
-                                                                    job.gstate, job.gact, c->adj_bnd.as<float>(), c->work.as<unsigned long long>());
-        c->launches++;
-        c->adjoint_launches++;
-        KS_CUDA(c, cudaGetLastError());
-    }
-    // the element phase
-    {
-        constexpr int W = NT / 32;
-        const long long grid = std::min<long long>(job.total / W + 1, (long long)nsm * per_sm);
-        const size_t smem = AdjSmem<CH>::bytes(ntot, W, global_acc);
-        k_adj_elements<CH, NT><<<unsigned(grid), NT, smem, c->stream>>>(c->st, job, c->tab32.as<float>(), c->gtab.as<double>(), ntot, dt, dn,
-                                                                       c->plan.as<double>(), c->stream_buf.as<float>(), job.gstate, job.gact,
-                                                                       c->work.as<unsigned long long>() + 1, c->adj_unit.as<float>(),
-                                                                       global_acc ? 1 : 0, c->errflag.as<unsigned>());
-        c->launches++;
-        c->adjoint_launches++;
-        KS_CUDA(c, cudaGetLastError());
-    }
-    const int per_chunk = 256;
-    const int nchunks = int((job.total + per_chunk - 1) / per_chunk);
-    KS_CUDA(c, c->adj_part.ensure(size_t(nchunks) * gsz * sizeof(double)));
-    k_unit_reduce1<<<dim3(nblocks(gsz, 128), nchunks), 128, 0, c->stream>>>(c->adj_unit.as<float>(), job.total, gsz, per_chunk,
-                                                                             c->adj_part.as<double>());
-    k_unit_reduce2<<<nblocks(gsz, 128), 128, 0, c->stream>>>(c->adj_part.as<double>(), nchunks, gsz, c->dgrad.as<double>());
-    c->launches += 2;
-    KS_CUDA(c, cudaGetLastError());
-    return KS_OK;
-}
-
-template <int CH>
-int launch_adjoint_mixed_ch(ks_context* c, int ntot, const double* dt, const double* dn) {
-    if (ntot > 32 * kMaxSplatWords) return fail(c, KS_ERR_ARGUMENT, "the mixed adjoint takes at most %d splats (%d)", 32 * kMaxSplatWords, ntot);
-    // the per-warp accumulator in shared memory while it leaves at least eight warps per SM, else the
-    // unit's block of global memory
-    // (384-thread blocks cap the element phase at 170 registers, with some spills, for 12 warps per SM
-    // instead of 8: 6% faster at configuration 3, the same sums)
-    bool global_acc = false;
-    int w384 = adjoint_blocks<CH, 384>(c, ntot, false) * 12, w256 = adjoint_blocks<CH, 256>(c, ntot, false) * 8,
-        w128 = adjoint_blocks<CH, 128>(c, ntot, false) * 4, w64 = adjoint_blocks<CH, 64>(c, ntot, false) * 2;
-    if (std::max(std::max(w384, w256), std::max(w128, w64)) < 8) {
-        global_acc = true;
-        w384 = adjoint_blocks<CH, 384>(c, ntot, true) * 12; w256 = adjoint_blocks<CH, 256>(c, ntot, true) * 8;
-        w128 = adjoint_blocks<CH, 128>(c, ntot, true) * 4; w64 = adjoint_blocks<CH, 64>(c, ntot, true) * 2;
-    }
-    const int best = std::max(std::max(w384, w256), std::max(w128, w64));
-    if (best <= 0) return fail(c, KS_ERR_ARGUMENT, "too many splats for the mixed adjoint (%d)", ntot);
-    if (w384 == best) return launch_adjoint_mixed_nt<CH, 384>(c, ntot, w384 / 12, dt, dn, global_acc);
-    if (w256 == best) return launch_adjoint_mixed_nt<CH, 256>(c, ntot, w256 / 8, dt, dn, global_acc);
-    if (w128 == best) return launch_adjoint_mixed_nt<CH, 128>(c, ntot, w128 / 4, dt, dn, global_acc);
-    return launch_adjoint_mixed_nt<CH, 64>(c, ntot, w64 / 2, dt, dn, global_acc);
 }
 
 // The forward image with the state the reverse pass needs (FP64: stored samples, cutoffs, tails),
@@ -2165,63 +1587,34 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
     const int N = c->st.N;
     const int ncombo = nframes * nfreq;
     const long long nrc = n * ncombo;
-    // the times, the frequencies (the mixed forward pass), then per combination fv * nframes + ft its
-    // time and frequency (the plain path)
-    std::vector<double> hc(ht);
+    std::vector<double> hc(ht);   // the times, then the frequencies
     hc.insert(hc.end(), hnu.begin(), hnu.end());
-    hc.resize(size_t(nframes) + nfreq + 2 * size_t(ncombo));
-    for (int fv = 0; fv < nfreq; ++fv)
-        for (int ft = 0; ft < nframes; ++ft) {
-            hc[nframes + nfreq + size_t(fv) * nframes + ft] = ht[ft];
-            hc[nframes + nfreq + ncombo + size_t(fv) * nframes + ft] = hnu[fv];
-        }
-    KS_CUDA(c, c->combos.ensure(hc.size() * sizeof(double)));
+    KS_CUDA(c, c->combos.ensure((size_t(nframes) + nfreq + 2 * size_t(ncombo)) * sizeof(double)));
     KS_CUDA(c, cudaMemcpyAsync(c->combos.p, hc.data(), hc.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    const double* dtimes = c->combos.as<double>();
-    const double* dfreqs = dtimes + nframes;
-    const double* dct = dfreqs + nfreq;
-    const double* dcn = dct + ncombo;
     KS_CUDA(c, c->out_sorted.ensure(size_t(nrc) * 4 * sizeof(double)));
     KS_CUDA(c, c->seeds.ensure(size_t(nrc) * 4 * sizeof(double)));
     KS_CUDA(c, c->dgrad.ensure(size_t(std::max(ntot, 1)) * GR_COUNT * sizeof(double)));
     cudaEventRecord(c->ev0, c->stream);
     const bool mixed = precision == KS_MIXED;
     // 1. forward pass with the reverse pass's state
-    StoredSamples S{};
-    const int* kst = nullptr;
-    const size_t tab_smem = size_t(ntot) * ST_COUNT * sizeof(double);
+    const long long piece = mixed ? n : plain_state_rays(c, nframes, nfreq);   // FP64: rays whose state is held at a time
     if (mixed) {
         c->geo64 = geo;
         const size_t rows = size_t(ncombo) * N * c->npad;
-        KS_CUDA(c, c->adj_state.ensure(rows * 27 * sizeof(float)));
+        KS_CUDA(c, c->adj_state.ensure(rows * 32 * sizeof(float)));
         KS_CUDA(c, c->adj_act.ensure(rows));
         KS_CUDA(c, cudaMemsetAsync(c->adj_act.p, 0, rows, c->stream));
         c->fwd_gstate = c->adj_state.as<float>();
         c->fwd_gact = c->adj_act.as<unsigned char>();
-        int s = launch_mixed(c, ntot, ht.data(), nframes, nfreq, L, nmax, slab, true);
+        int s = launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, true);
         c->fwd_gstate = nullptr;
         c->fwd_gact = nullptr;
         if (s) return s;
     } else {
-    if (tab_smem > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for the FP64 adjoint (%d)", ntot);
-    {
-        int s = ensure_samples(c, &S);
+        if (size_t(ntot) * ST_COUNT * sizeof(double) > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for the FP64 adjoint (%d)", ntot);
+        int s = piece >= n ? launch_plain_state(c, ntot, nframes, nfreq, L, nmax, slab, 0, n)
+                           : launch_plain(c, ntot, nframes, nfreq, L, nmax, slab, true);
         if (s) return s;
-    }
-    if (nmax >= 0) {
-        KS_CUDA(c, c->kstop.ensure(size_t(n) * sizeof(int)));
-        k_kstop<<<nblocks(n), kBlock, 0, c->stream>>>(S, n, N, c->st.rh * (1 + 1e-3), nmax, slab, c->kstop.as<int>());
-        c->launches++;
-        KS_CUDA(c, cudaGetLastError());
-        kst = c->kstop.as<int>();
-    }
-    KS_CUDA(c, c->tails.ensure(size_t(ncombo) * (N + 1) * 4 * n * sizeof(double)));
-    KS_CUDA(c, cudaFuncSetAttribute(k_tails, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_smem));
-    k_tails<<<nblocks(nrc), kBlock, tab_smem, c->stream>>>(plan_view(c), c->st, n, S, kst, c->tab.as<double>(), ntot, dct, dcn, ncombo, L,
-                                                          c->tails.as<double>(), c->out_sorted.as<double>());
-    c->launches++;
-    c->adjoint_launches++;
-    KS_CUDA(c, cudaGetLastError());
     }
     // 2. seeds
     const long long nblk = (nrc + 255) / 256;
@@ -2294,32 +1687,14 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
     }
     // 3. reverse pass and the deterministic reduction
     if (ntot > 0 && mixed) {
-        // the reverse pass groups frequencies as the forward pass did
-        const int ch = c->last_job.ch;
-        int s = ch == 4 ? launch_adjoint_mixed_ch<4>(c, ntot, dtimes, dfreqs)
-                        : (ch == 3 ? launch_adjoint_mixed_ch<3>(c, ntot, dtimes, dfreqs)
-                                   : (ch == 2 ? launch_adjoint_mixed_ch<2>(c, ntot, dtimes, dfreqs) : launch_adjoint_mixed_ch<1>(c, ntot, dtimes, dfreqs)));
+        int s = launch_reverse(c, ntot, nmax, false, false);
         if (s) return s;
     } else if (ntot > 0) {
-        // per-ray slots in ray chunks of at most 4 GB, each reduced (in ray order) into dgrad
-        const long long per_ray = (long long)GR_COUNT * ntot * ncombo * (long long)sizeof(double);
-        const long long nr = std::max(1LL, std::min(n, (4LL << 30) / per_ray));
-        KS_CUDA(c, c->slots.ensure(size_t(nr) * per_ray));
-        KS_CUDA(c, cudaFuncSetAttribute(k_dual_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_smem));
-        for (long long j0 = 0; j0 < n; j0 += nr) {
-            const long long m = std::min(nr, n - j0);
-            KS_CUDA(c, cudaMemsetAsync(c->slots.p, 0, size_t(m) * per_ray, c->stream));
-            k_dual_plain<<<nblocks(m * ncombo), kBlock, tab_smem, c->stream>>>(plan_view(c), c->st, n, S, kst, c->tab.as<double>(),
-                                                                              c->gtab.as<double>(), ntot, dct, dcn, ncombo, L,
-                                                                              c->tails.as<double>(), c->seeds.as<double>(),
-                                                                              c->slots.as<double>(), j0, m);
-            c->launches++;
-            c->adjoint_launches++;
-            KS_CUDA(c, cudaGetLastError());
-            k_slot_reduce<<<unsigned(GR_COUNT * ntot), 256, 0, c->stream>>>(c->slots.as<double>(), m * ncombo, ntot, c->dgrad.as<double>(),
-                                                                            j0 > 0 ? 1 : 0);
-            c->launches++;
-            KS_CUDA(c, cudaGetLastError());
+        for (long long j0 = 0; j0 < n; j0 += piece) {
+            int s = KS_OK;
+            if (piece < n) s = launch_plain_state(c, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, n - j0));
+            if (s == KS_OK) s = launch_reverse(c, ntot, nmax, true, j0 > 0);
+            if (s) return s;
         }
     }
     cudaEventRecord(c->ev1, c->stream);
@@ -2401,9 +1776,6 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
     const long long nrc = n * ncombo;
     const long long nblk = (nrc + 255) / 256;
     const size_t rows = size_t(ncombo) * c->st.N * c->npad;
-    const double* dtimes = c->combos.as<double>();   // as the ordinary evaluation wrote them
-    const double* dfreqs = dtimes + nframes;
-    const int ch = c->last_job.ch;
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
     status = capture_tables(c, sets, nsets, ntot, true);
@@ -2413,7 +1785,7 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
         if (cudaMemsetAsync(c->adj_act.p, 0, rows, c->stream) != cudaSuccess) status = fail(c, KS_ERR_DEVICE, "graph capture: activity reset");
         c->fwd_gstate = c->adj_state.as<float>();
         c->fwd_gact = c->adj_act.as<unsigned char>();
-        if (status == KS_OK) status = launch_mixed(c, ntot, nullptr, nframes, nfreq, L, nmax, slab, true);
+        if (status == KS_OK) status = launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, true);
         c->fwd_gstate = nullptr;
         c->fwd_gact = nullptr;
     }
@@ -2424,9 +1796,7 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
         if (cudaGetLastError() != cudaSuccess) status = fail(c, KS_ERR_DEVICE, "graph capture: chi^2 seeds");
     }
     if (status == KS_OK && ntot > 0)
-        status = ch == 4 ? launch_adjoint_mixed_ch<4>(c, ntot, dtimes, dfreqs)
-                         : (ch == 3 ? launch_adjoint_mixed_ch<3>(c, ntot, dtimes, dfreqs)
-                                    : (ch == 2 ? launch_adjoint_mixed_ch<2>(c, ntot, dtimes, dfreqs) : launch_adjoint_mixed_ch<1>(c, ntot, dtimes, dfreqs)));
+        status = launch_reverse(c, ntot, nmax, false, false);
     const long long ng = (long long)ntot * GR_COUNT;
     if (status == KS_OK && ng > 0) {
         k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate);
@@ -2765,11 +2135,11 @@ int ks_autotune(ks_context* c, const ks_splat_set* sets, int32_t nsets, const do
     const long long n4 = c->npix * (long long)nframes * nfreq * 4;
     if (nframes < 1 || nfreq < 1) return fail(c, KS_ERR_ARGUMENT, "need at least one frame and one frequency");
     KS_CUDA(c, c->st_buf.ensure(size_t(n4) * sizeof(double)));
-    const int cand_nt[3] = {384, 256, 128}, cand_u[4] = {2, 4, 8, 16};
+    const int cand_nt[2] = {256, 128}, cand_u[4] = {2, 4, 8, 16};
     double best = 1e300;
     int bnt = 0, bu = 0;
     const int save_nt = c->tune_nt, save_u = c->tune_units;
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 2; ++a)
         for (int b = 0; b < 4; ++b) {
             c->tune_nt = cand_nt[a]; c->tune_units = cand_u[b];
             int s = ks_render(c, sets, nsets, times, nframes, nus, nfreq, L, KS_MIXED, nmax, slab, c->st_buf.as<double>(), KS_ORDER_SORTED);

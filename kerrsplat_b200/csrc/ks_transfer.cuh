@@ -421,9 +421,9 @@ __device__ __forceinline__ LFrame<T> local_frame(const SampleFrame<T>& F, T u1, 
 
 // ---- step.jl --------------------------------------------------------------------------------------
 
-// M_n(a) = int_0^1 t^n e^{-at} dt for n = 0..9 (step.jl:239-268); the series coefficients
+// M_n(a) = int_0^1 t^n e^{-at} dt for n = 0..10 (step.jl:239-268); the series coefficients
 // (-1)^m / (m! (n + m + 1)) are generated on the host into constant memory.
-struct MomentCoeffs { double c[10][24]; float cf[10][24]; };
+struct MomentCoeffs { double c[11][24]; float cf[11][24]; };
 
 template <class T>
 __device__ __forceinline__ T mcoef(const MomentCoeffs& MC, int n, int m) {
@@ -463,7 +463,7 @@ __device__ __forceinline__ void moments(const MomentCoeffs& MC, T a, T M[10]) {
 }
 // FP32: one out-of-line copy; for |a| < 1 the series of M_9 and the downward recurrence
 // M_{n-1} = (a M_n + e^{-a}) / n, stable for |a| < 1 (each step scales the error by |a| / n)
-__device__ __noinline__ void moments_f32(const MomentCoeffs& MC, float a, float* M) {
+static __device__ __noinline__ void moments_f32(const MomentCoeffs& MC, float a, float* M) {
     if (fabsf(a) < 1.f) {
         float s = MC.cf[9][23];
 #pragma unroll
@@ -480,6 +480,29 @@ __device__ __noinline__ void moments_f32(const MomentCoeffs& MC, float a, float*
     }
 }
 template <> __device__ __forceinline__ void moments<float>(const MomentCoeffs& MC, float a, float M[10]) { moments_f32(MC, a, M); }
+// Duals: the values M_0..M_10 by the downward recurrence from the series of M_10 (|a| < 1) or the upward one, and
+// dM_n/da = -M_{n+1}
+template <class T, int N>
+__device__ __forceinline__ void moments(const MomentCoeffs& MC, Dual<T, N> a, Dual<T, N> M[10]) {
+    T m[11];
+    const T e = fexp(-a.v);
+    if (fabs(a.v) < T(1)) {
+        constexpr int K = is_f32<T> ? 11 : 23;
+        T s = mcoef<T>(MC, 10, K);
+#pragma unroll
+        for (int q = K - 1; q >= 0; --q) s = fma(a.v, s, mcoef<T>(MC, 10, q));
+        m[10] = s;
+#pragma unroll
+        for (int n = 10; n >= 1; --n) m[n - 1] = (a.v * m[n] + e) * T(1.0 / n);
+    } else {
+        const T ia = T(1) / a.v;
+        m[0] = (T(1) - e) * ia;
+#pragma unroll
+        for (int n = 1; n < 11; ++n) m[n] = (T(n) * m[n - 1] - e) * ia;
+    }
+#pragma unroll
+    for (int n = 0; n < 10; ++n) M[n] = dchain(a, m[n], -m[n + 1]);
+}
 
 template <class T> __device__ __forceinline__ T phi_fn(const MomentCoeffs& MC, T a) {
     if (fabs(a) < T(1)) return moment_n(MC, a, 0);
@@ -769,6 +792,24 @@ __device__ __forceinline__ void transfer_step_structured(const MomentCoeffs& MC,
 #pragma unroll
     for (int i = 0; i < 4; ++i) E[i] = s * (e[0] * j4[i] + e[1] * Kj[i] + e[2] * K2j[i] + e[3] * K3j[i]);
 }
+
+// ---- coordinates ------------------------------------------------------------------------------------
+
+// The quasi-Cartesian Kerr-Schild position of a Boyer-Lindquist point (coordinates.jl:22-31).
+template <class T>
+__device__ __forceinline__ void ks_position(T a, T r, T sth, T cth, T ph, T& x, T& y, T& z) {
+    T temp = sqrt(T(1) - a * a);
+    T rp = T(1) + temp, rm = T(1) - temp;
+    T phks = ph + a / (T(2) * temp) * log(fabs((r - rp + keps<T>()) / (r - rm + keps<T>()))) - atan2(a, r);
+    T sp = sin(phks), cp = cos(phks);
+    x = r * sth * cp; y = r * sth * sp; z = r * cth;
+}
+template <class T>
+__device__ __forceinline__ void ks_coords(T a, T r, T th, T ph, T& x, T& y, T& z, T& sth, T& cth) {
+    sth = sin(th); cth = cos(th);
+    ks_position(a, r, sth, cth, ph, x, y, z);
+}
+
 
 // ---- splats -------------------------------------------------------------------------------------
 
