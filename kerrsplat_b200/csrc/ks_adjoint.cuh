@@ -323,21 +323,21 @@ __global__ void __launch_bounds__(64) k_jvp(PlanView P, Spacetime st, long long 
     }
 }
 
-// The mixed J v over the FP32 sample stream of k_stream (the FP64 march rounded to FP32, the
-// Kerr-Schild position formed there: the samples k_jvp<float, K> would round its own march to) instead
-// of a march per thread; one thread per (ray, combination), outputs as k_jvp. At most 128 registers
-// (16 warps per SM instead of 12 at 168; 4% faster on configuration-5 sets, the same J v).
+// The mixed J v over the FP32 sample stream of k_stream: one thread per (segment of the samples, combination, ray),
+// which composes the segment's (P, S) on duals; k_jvp_combine joins the segments. Bound by the dual pair evaluations
+// of the rays that cross splats: one thread per whole ray ran 71 ms for two directions on 96 x 96 rays x 256 samples,
+// two warps per SM deep. The first sample past the half-orbit cutoff is `kstop` (null: none).
 template <int K>
 __global__ void __launch_bounds__(64, 8) k_jvp_stream(PlanView P, Spacetime st, long long npix, const Dual<float, K>* __restrict__ dtab, int ntot,
-                                                   const double* __restrict__ ct, const double* __restrict__ cnu, int ncombo, double L, int nmax,
-                                                   double slab, const float* __restrict__ stream, double* __restrict__ img, double* __restrict__ out,
-                                                   int lnL_dir) {
+                                                   const double* __restrict__ ct, const double* __restrict__ cnu, int ncombo, double L,
+                                                   const int* __restrict__ kstop, int nseg, int seg_len, const float* __restrict__ stream,
+                                                   float* __restrict__ part, int lnL_dir) {
     __shared__ float s_reach;
     const float reach2 = table_reach2(dtab, ntot, &s_reach);   // before any thread leaves: it has block barriers
     const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= npix * ncombo) return;
+    if (idx >= npix * ncombo * nseg) return;
     const long long j = idx % npix;
-    const int c = int(idx / npix);
+    const int c = int(idx / npix % ncombo), seg = int(idx / npix / ncombo);
     const long long npad = P.npad;
     JvpSink<float, K> sink;
     sink.tab = dtab; sink.ntot = ntot; sink.reach2 = reach2;
@@ -347,20 +347,54 @@ __global__ void __launch_bounds__(64, 8) k_jvp_stream(PlanView P, Spacetime st, 
     sink.a = float(st.a); sink.rh_lo = float(st.rh * (1 + 1e-3)); sink.dtau = float(P.get(PF_DTAU, j));
     sink.alpha = float(P.get(PF_ALPHA, j)); sink.beta = float(P.get(PF_BETA, j));
     sink.eta = float(P.get(PF_ETA, j)); sink.lam = float(P.get(PF_LAM, j));
-    sink.a_sin_tho = float(st.a * sin(st.thetao)); sink.slab = float(slab); sink.nmax = nmax;
+    sink.a_sin_tho = float(st.a * sin(st.thetao)); sink.slab = 0.f; sink.nmax = -1;
     sink.lnL_dir = lnL_dir;
     sink.init();
-    const int Nj = int(P.get(PF_NSAMP, j));
-    const float* sp = stream + j;
-    for (int k = 1; k <= Nj; ++k, sp += SM_COUNT * npad) {
+    int k1 = min(int(P.get(PF_NSAMP, j)) + 1, 1 + (seg + 1) * seg_len);
+    if (kstop) k1 = min(k1, kstop[j]);
+    const float* sp = stream + (long long)seg * seg_len * SM_COUNT * npad + j;
+    for (int k = 1 + seg * seg_len; k < k1; ++k, sp += SM_COUNT * npad) {
         const unsigned flags = __float_as_uint(sp[SM_FLAGS * npad]);
         sink.stream_sample((flags & 8u) != 0u, sp[SM_X * npad], sp[SM_Y * npad], sp[SM_Z * npad], sp[SM_T * npad], sp[SM_R * npad],
                            sp[SM_STH * npad], sp[SM_CTH * npad], (flags & 2u) != 0u, (flags & 4u) != 0u);
     }
-    const double n3 = nh * nh * nh;
-    for (int s = 0; s < 4; ++s) {
-        img[(c * npix + j) * 4 + s] = double(sink.Sv[s].v) * n3;
-        for (int d = 0; d < K; ++d) out[(((long long)d * ncombo + c) * npix + j) * 4 + s] = double(sink.Sv[s].d[d]) * n3;
+    // [seg][combination][20 (K + 1)][ray]
+    float* o = part + (idx / npix) * (20 * (K + 1)) * npix + j;
+    for (int q = 0; q < 20; ++q) {
+        const Dual<float, K>& x = q < 16 ? sink.P[q] : sink.Sv[q - 16];
+        o[(long long)q * (K + 1) * npix] = x.v;
+        for (int d = 0; d < K; ++d) o[(long long)(q * (K + 1) + 1 + d) * npix] = x.d[d];
+    }
+}
+
+// The segments of a ray front to back (S = S_0 + P_0 (S_1 + ...)) on duals, and the observed Stokes vector (x nuhat^3).
+template <int K>
+__global__ void k_jvp_combine(long long npix, int ncombo, int nseg, const double* __restrict__ cnu, const float* __restrict__ part,
+                              double* __restrict__ img, double* __restrict__ out) {
+    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (idx >= npix * ncombo) return;
+    const long long j = idx % npix, c = idx / npix;
+    double S[4][K + 1];
+    for (int r = 0; r < 4; ++r)
+        for (int d = 0; d <= K; ++d) S[r][d] = 0.0;
+    for (int sg = nseg - 1; sg >= 0; --sg) {
+        const float* p = part + ((long long)sg * ncombo + c) * (20 * (K + 1)) * npix + j;
+        double T[4][K + 1];
+        for (int r = 0; r < 4; ++r) {
+            for (int d = 0; d <= K; ++d) T[r][d] = p[(long long)((16 + r) * (K + 1) + d) * npix];
+            for (int q = 0; q < 4; ++q) {
+                const double pv = p[(long long)((4 * r + q) * (K + 1)) * npix];
+                T[r][0] += pv * S[q][0];
+                for (int d = 1; d <= K; ++d) T[r][d] += pv * S[q][d] + double(p[(long long)((4 * r + q) * (K + 1) + d) * npix]) * S[q][0];
+            }
+        }
+        for (int r = 0; r < 4; ++r)
+            for (int d = 0; d <= K; ++d) S[r][d] = T[r][d];
+    }
+    const double nh = cnu[c] / kNU0, n3 = nh * nh * nh;
+    for (int r = 0; r < 4; ++r) {
+        img[(c * npix + j) * 4 + r] = S[r][0] * n3;
+        for (int d = 0; d < K; ++d) out[(((long long)d * ncombo + c) * npix + j) * 4 + r] = S[r][1 + d] * n3;
     }
 }
 

@@ -47,7 +47,7 @@ struct ks_context {
     // adjoint: gradient table, stored FP64 samples (plain path), cutoffs, tails, per-ray slots,
     // seeds, chi^2 partials; mixed path: per-sample states, activity, segment bounds, unit partials
     DevBuf gtab, samples, kstop, dgrad, seeds, chi_part, chi_val, dstage;
-    DevBuf adj_state, adj_act, adj_bnd, adj_unit, adj_part, jvp_tab, jvp_in, jvp_out, st_buf;
+    DevBuf adj_state, adj_act, adj_bnd, adj_unit, adj_part, jvp_tab, jvp_in, jvp_out, jvp_part, st_buf;
     DevBuf rows;      // the transport's splat rows and knot array (FP32 or FP64)
     DevBuf stream64, seg_out64;   // the FP64 render's stream and segment states
     DevBuf tab32;     // the splat table and knot array in FP32, padded to 16 bytes (the TMA staging source)
@@ -141,6 +141,8 @@ inline ks::PlanView plan_view(ks_context* c) {
 int forward_init(const ks::MomentCoeffs& mc);
 // The FP32 sample stream of every ray.
 int launch_stream(ks_context* c);
+// The half-orbit cutoff of every ray on the FP32 stream, into c->kstop.
+int launch_wind_stop(ks_context* c, int nmax, double slab);
 // The render into c->out_sorted from the tables that build_tables left: FP32 transport over the FP32 stream, or
 // FP64 throughout. The times, then the frequencies, lie in c->combos.
 int launch_mixed(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only);

@@ -39,6 +39,15 @@ int launch_stream(ks_context* c) {
     return KS_OK;
 }
 
+int launch_wind_stop(ks_context* c, int nmax, double slab) {
+    KS_CUDA(c, c->kstop.ensure(size_t(c->npix) * sizeof(int)));
+    k_wind_stop<float><<<nblocks(c->npix), kBlock, 0, c->stream>>>(plan_view(c), 0, c->npix, c->npad, c->stream_buf.as<float>(), nmax, float(slab),
+                                                                  c->kstop.as<int>());
+    c->launches++;
+    KS_CUDA(c, cudaGetLastError());
+    return KS_OK;
+}
+
 // How a transport kernel of NT threads is shaped for a scene: samples per run, records per window, blocks per SM.
 struct Shape {
     int run = 0, cap = 0, blocks = 0;
@@ -135,11 +144,7 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     if (s || (s = build_rows<float, KM>(c, ntot, c->fwd_gstate != nullptr))) return s;
     TransportJob job = transport_job(c, ntot, nframes, nfreq, CH, L, 0, c->npix, c->npad);
     if (nmax >= 0) {
-        KS_CUDA(c, c->kstop.ensure(size_t(c->npix) * sizeof(int)));
-        k_wind_stop<float><<<nblocks(c->npix), kBlock, 0, c->stream>>>(plan_view(c), 0, c->npix, c->npad, c->stream_buf.as<float>(), nmax,
-                                                                      float(slab), c->kstop.as<int>());
-        c->launches++;
-        KS_CUDA(c, cudaGetLastError());
+        if ((s = launch_wind_stop(c, nmax, slab))) return s;
         job.kstop = c->kstop.as<int>();
     }
     constexpr int B128 = 4, B256 = 2;

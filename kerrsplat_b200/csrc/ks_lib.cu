@@ -1856,10 +1856,23 @@ int jvp_chunk(ks_context* c, int ntot, const double* dparams_dev, const double* 
         KS_CUDA(c, cudaGetLastError());
     }
     const long long nrc = c->npix * ncombo;
-    if constexpr (std::is_same<S, float>::value)
-        k_jvp_stream<K><<<nblocks(nrc, 64), 64, 0, c->stream>>>(plan_view(c), c->st, c->npix, dt, ntot, dct, dcn, ncombo, L, nmax, slab,
-                                                                c->stream_buf.as<float>(), img_sorted, out_sorted, lnL_dir);
-    else
+    if constexpr (std::is_same<S, float>::value) {
+        // segments until there are some 32 warps per SM (at least 16 samples each), as far as 4 GB of segment states go
+        int nseg = 1;
+        while (nrc * nseg < 148LL * 1024 && (nseg * 2) * 16 <= c->st.N && nrc * nseg * 2 * 20 * (K + 1) * (long long)sizeof(float) <= (4LL << 30)) nseg *= 2;
+        const int seg_len = (c->st.N + nseg - 1) / nseg;
+        KS_CUDA(c, c->jvp_part.ensure(size_t(nrc) * nseg * 20 * (K + 1) * sizeof(float)));
+        const int* kstop = nullptr;
+        if (nmax >= 0) {
+            int s = launch_wind_stop(c, nmax, slab);
+            if (s) return s;
+            kstop = c->kstop.as<int>();
+        }
+        k_jvp_stream<K><<<nblocks(nrc * nseg, 64), 64, 0, c->stream>>>(plan_view(c), c->st, c->npix, dt, ntot, dct, dcn, ncombo, L, kstop, nseg, seg_len,
+                                                                       c->stream_buf.as<float>(), c->jvp_part.as<float>(), lnL_dir);
+        k_jvp_combine<K><<<nblocks(nrc, 128), 128, 0, c->stream>>>(c->npix, ncombo, nseg, dcn, c->jvp_part.as<float>(), img_sorted, out_sorted);
+        c->launches++;
+    } else
         k_jvp<S, K><<<nblocks(nrc, 64), 64, 0, c->stream>>>(plan_view(c), c->st, c->npix, dt, ntot, dct, dcn, ncombo, L, nmax, slab, img_sorted,
                                                             out_sorted, lnL_dir);
     c->launches++;
@@ -1911,7 +1924,8 @@ int jvp_impl(ks_context* c, const ks_splat_set* sets, int32_t nsets, const doubl
             off += cnt;
         }
     }
-    const int K = ndir == 1 ? 1 : 8;
+    // directions of a pass: the FP32 pass carries no more partials than there are directions
+    const int K = ndir == 1 ? 1 : precision == KS_FP64 || ndir > 4 ? 8 : ndir == 2 ? 2 : 4;
     const int nchunk = (ndir + K - 1) / K;
     // directions padded to whole chunks
     std::vector<double> hd(size_t(nchunk) * K * np, 0.0);
@@ -1951,7 +1965,9 @@ int jvp_impl(ks_context* c, const ks_splat_set* sets, int32_t nsets, const doubl
                        : jvp_chunk<double, 8>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld);
         else
             s = K == 1 ? jvp_chunk<float, 1>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld)
-                       : jvp_chunk<float, 8>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld);
+                       : K == 2 ? jvp_chunk<float, 2>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld)
+                       : K == 4 ? jvp_chunk<float, 4>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld)
+                                : jvp_chunk<float, 8>(c, ntot, dp, dd, np, dct, dcn, ncombo, L, nmax, slab, c->out_sorted.as<double>(), c->jvp_out.as<double>(), ld);
         if (s) return s;
         const int nd = std::min(K, ndir - ch * K);
         s = emit(c, c->jvp_out.as<double>(), 4, int(nd * ncombo), order, dimage + (long long)ch * K * nrc * 4);
