@@ -49,6 +49,7 @@ struct ks_context {
     DevBuf gtab, samples, kstop, dgrad, seeds, chi_part, chi_val, dstage;
     DevBuf adj_state, adj_act, adj_bnd, adj_unit, adj_part, jvp_tab, jvp_in, jvp_out, jvp_part, st_buf;
     DevBuf rows;      // the transport's splat rows and knot array (FP32 or FP64)
+    DevBuf thin_part;             // the thin image's pieces (sized by regenerate)
     DevBuf stream64, seg_out64;   // the FP64 render's stream and segment states
     DevBuf tab32;     // the splat table and knot array in FP32, padded to 16 bytes (the TMA staging source)
     DevBuf errflag;   // set by a kernel whose bounded wait gave up
@@ -64,7 +65,6 @@ struct ks_context {
     int tune_nt = 0, tune_units = 0;        // the autotuner's choice for the mixed forward (0: the default)
     int nkv = 0;                            // knot values after the splat table in `tab`
     ks::TransportJob last_job{};            // the last forward pass with an adjoint's state
-    long long state_rays = 0;               // FP64 adjoint: rays per piece whose state is held
     float* fwd_gstate = nullptr;            // set during the adjoint's forward pass only
     unsigned char* fwd_gact = nullptr;
     double adjoint_ms = 0.0;

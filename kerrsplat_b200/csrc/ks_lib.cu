@@ -4,11 +4,11 @@
 // Pipeline of one context (the device-side GeodesicCache of cache.jl:85-125):
 //   ks_regenerate: k_root_case (K0, screen order) -> stable radix sort by root case (4, 2, 0 real
 //     roots; cub, deterministic) -> k_build_plan (K1: FP64 per-ray constants, sorted order) ->
-//     exclusive scan of anchor counts -> k_anchor_segments (one thread per (ray, anchor): Jacobi
-//     states, validity, closed-form parts and the Gauss-Legendre integral of the smooth part since
-//     the previous anchor) -> k_anchor_prefix (per-ray running sums).
-//   ks_thin_image / ks_render: k_splat_table (per-splat FP64 constants) -> k_thin / k_transport
-//     (one thread per ray, the fused march with the consumer folded over the samples) -> k_unsort.
+//     exclusive scan of anchor counts -> k_anchor_segments (one thread per two anchors of a ray: Jacobi
+//     states by the addition theorem, validity, closed-form parts and the Gauss-Legendre integral of the
+//     smooth part since the previous anchor) -> k_anchor_prefix (per-ray running sums).
+//   ks_thin_image / ks_render: k_splat_table (per-splat FP64 constants) -> k_thin (a block marches 32 rays,
+//     in pieces of their depth) or k_stream -> k_transport -> k_compose (ks_transport.cuh) -> k_unsort.
 #include <cub/cub.cuh>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -477,10 +477,18 @@ __global__ void k_march_store(PlanView P, Spacetime st, long long npix, double* 
     resid_t[j] = rt; resid_phi[j] = rp;
 }
 
-// ThinRenderer (Splats.jl:113-128)
+// ThinRenderer (Splats.jl:113-128) over rows of kThinRow values: the centre, t0, omega, 1 / w, ln A, and the whitened
+// rotation R diag(exp(-s)) formed in FP64.
+constexpr int kThinRow = 16;
+template <class T>
+__device__ __forceinline__ T thin_row(const double* p, int f) {
+    constexpr int head[7] = {ST_CX, ST_CY, ST_CZ, ST_T0, ST_OMEGA, ST_INVW, ST_LOGA};
+    return f < 7 ? T(p[head[f]]) : T(p[ST_R0 + f - 7] * p[ST_ES1 + (f - 7) % 3]);
+}
+
 template <class T>
 struct ThinSink {
-    const T* tab; int nsplat; T t_obs; T a, rh_lo; T dtau; T acc;
+    const T* rows; int nsplat; T t_obs; T a, rh_lo; T dtau; T acc;
     T eta, lam;
     __device__ void operator()(int, const Sample<T>& s) {
         if (!(s.ok && rh_lo < s.r && s.r < T(1e3))) return;
@@ -488,61 +496,80 @@ struct ThinSink {
         const T cth = s.cos_theta, sth = sqrt(fmax((T(1) - cth) * (T(1) + cth), T(0)));
         T x, y, z;
         ks_position(a, s.r, sth, cth, s.phi, x, y, z);
-        T t = t_obs - s.t;
+        const T t = t_obs - s.t;
         T jt = T(0);
         for (int i = 0; i < nsplat; ++i) {
-            const T* p = tab + i * ST_COUNT;
-            T q;
-            splat_exponent(p, t, x, y, z, false, q);
-            jt += exp(p[ST_LOGA] - q);
+            const T* p = rows + i * kThinRow;
+            const T dt = t - p[3];
+            T sp, cp;
+            fsincos(p[4] * dt, sp, cp);
+            const T d0 = x - (p[0] * cp - p[1] * sp), d1 = y - (p[0] * sp + p[1] * cp), d2 = z - p[2];
+            const T b0 = d0 * cp + d1 * sp, b1 = -d0 * sp + d1 * cp;
+            const T e0 = p[7] * b0 + p[10] * b1 + p[13] * d2, e1 = p[8] * b0 + p[11] * b1 + p[14] * d2, e2 = p[9] * b0 + p[12] * b1 + p[15] * d2;
+            const T tt = dt * p[5];
+            jt += exp(p[6] - (e0 * e0 + e1 * e1 + e2 * e2 + tt * tt) / T(2));
         }
-        SampleFrame<T> F = sample_frame(a, s.r, s.theta, sth, cth, eta, lam, s.nur, s.nutheta);
+        SampleFrame<T> F = sample_frame(a, s.r, T(0), sth, cth, eta, lam, s.nur, s.nutheta);
         T g = T(1) / F.pz[0];
         T Sg = s.r * s.r + a * a * cth * cth;
         acc += g * g * jt * Sg * dtau;
     }
 };
 
-// The thin image: a ray is marched in nseg pieces (a power of two), one thread each, the threads of a
-// piece side by side, so that a warp's threads are neighbouring rays at the same depth; the pieces' sums (and anchor residuals) meet in shared memory in depth order. Bound by the
-// latency of the FP64 march (every sample is a chain of logarithms, arctangents and divisions): one
-// thread per ray kept 4 warps per SM at 128 x 128 rays.
+// The thin image: a block marches 32 rays (march_block), each thread taking a quarter of their samples, over one of
+// nseg pieces of their depth. One piece writes the image; with more, each leaves its sums (and anchor residuals) in
+// `part` [3][nseg][npix] for k_thin_sum. Bound by FP64 arithmetic on a full screen (every sample rotates every splat's
+// centre and exponentiates) and by the latency of the march on a small one. Whole calls, one thread a ray against these
+// blocks: 24 x 24 rays x 64 samples x 3 splats 560 : 260 us, 128 x 128 x 512 x 12 splats 6.09 : 2.49 ms.
 template <class T>
-__global__ void k_thin(PlanView P, Spacetime st, long long npix, const double* __restrict__ tab64, int nsplat, double t_obs, int nseg,
-                       const long long* __restrict__ perm, double* __restrict__ out, double* __restrict__ resid_t,
-                       double* __restrict__ resid_phi) {
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3)
+k_thin(PlanView P, Spacetime st, long long npix, const double* __restrict__ tab64, int nsplat, double t_obs, int nseg, double* __restrict__ part,
+       const long long* __restrict__ perm, double* __restrict__ out, double* __restrict__ resid_t, double* __restrict__ resid_phi) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double part[3][kBlock];
-    T* tab = reinterpret_cast<T*>(smem);
-    for (int q = threadIdx.x; q < nsplat * ST_COUNT; q += blockDim.x) tab[q] = T(tab64[q]);
+    __shared__ double red[kMarchWarps][32];
+    MarchShared<T>& shared = *reinterpret_cast<MarchShared<T>*>(smem);
+    T* rows = reinterpret_cast<T*>(smem + (sizeof(MarchShared<T>) + 15) / 16 * 16);
+    for (int q = threadIdx.x; q < nsplat * kThinRow; q += kBlock) rows[q] = thin_row<T>(tab64 + (q / kThinRow) * ST_COUNT, q % kThinRow);
+    const int lane = threadIdx.x & 31, seg = blockIdx.y;
+    const bool live = blockIdx.x * 32LL + lane < npix;
+    const long long j = live ? blockIdx.x * 32LL + lane : npix - 1;
+    const int nsamp = int(P.get(PF_NSAMP, j));
+    // pieces of whole re-anchoring intervals: each starts from the anchor table
+    const int len = ((nsamp + nseg - 1) / nseg + st.M - 1) / st.M * st.M;
+    ThinSink<T> sink{rows, nsplat, T(t_obs), T(st.a), T(st.rh * (1 + 1e-3)), T(P.get(PF_DTAU, j)), T(0), T(P.get(PF_ETA, j)), T(P.get(PF_LAM, j))};
+    double rt, rp;
+    march_block<true>(P, st, j, live, 1 + seg * len, 1 + (seg + 1) * len, shared, sink, rt, rp);   // its first barrier is behind the rows
+    red[threadIdx.x >> 5][lane] = double(sink.acc);
     __syncthreads();
-    const int nr = kBlock / nseg, seg = threadIdx.x / nr;
-    const long long j = blockIdx.x * (long long)nr + threadIdx.x % nr;
-    double rt = 0.0, rp = 0.0, acc = 0.0;
-    if (j < npix) {
-        MarchRay<T> R = load_ray<T>(P, st, j);
-        ThinSink<T> sink{tab, nsplat, T(t_obs), T(st.a), T(st.rh * (1 + 1e-3)), T(R.dtau), T(0), R.eta, R.lam};
-        // pieces of whole re-anchoring intervals: each starts from the anchor table
-        const int len = ((R.nsamp + nseg - 1) / nseg + st.M - 1) / st.M * st.M;
-        march_part(P, j, R, sink, 1 + seg * len, 1 + (seg + 1) * len, rt, rp);
-        acc = double(sink.acc);
-    }
-    part[0][threadIdx.x] = acc; part[1][threadIdx.x] = rt; part[2][threadIdx.x] = rp;
-    __syncthreads();
-    if (seg > 0 || j >= npix) return;
-    for (int s = 1; s < nseg; ++s) {
-        acc += part[0][threadIdx.x + s * nr];
-        rt = fmax(rt, part[1][threadIdx.x + s * nr]);
-        rp = fmax(rp, part[2][threadIdx.x + s * nr]);
+    if (threadIdx.x >= 32 || !live) return;
+    double acc = 0.0;
+    for (int w = 0; w < kMarchWarps; ++w) acc += red[w][lane];
+    if (nseg > 1) {
+        part[seg * npix + j] = acc; part[(nseg + seg) * npix + j] = rt; part[(2 * nseg + seg) * npix + j] = rp;
+        return;
     }
     out[perm ? perm[j] : j] = acc;   // sorted order, or screen order through the permutation
     if (resid_t) { resid_t[j] = rt; resid_phi[j] = rp; }
 }
 
-// Pieces per ray: one for each re-anchoring interval, up to 16 (a power of two).
-int thin_pieces(const Spacetime& st) {
+__global__ void k_thin_sum(long long npix, int nseg, const double* __restrict__ part, const long long* __restrict__ perm, double* __restrict__ out,
+                           double* __restrict__ resid_t, double* __restrict__ resid_phi) {
+    const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (j >= npix) return;
+    double acc = 0.0, rt = 0.0, rp = 0.0;
+    for (int s = 0; s < nseg; ++s) {
+        acc += part[s * npix + j];
+        rt = fmax(rt, part[(nseg + s) * npix + j]);
+        rp = fmax(rp, part[(2 * nseg + s) * npix + j]);
+    }
+    out[perm ? perm[j] : j] = acc;
+    if (resid_t) { resid_t[j] = rt; resid_phi[j] = rp; }
+}
+
+// Pieces of a screen's depth: until there are four blocks per SM, down to one re-anchoring interval each (up to 16).
+int thin_pieces(const Spacetime& st, long long npix) {
     int nseg = 1;
-    while (nseg < 16 && 2 * nseg * (long long)st.M <= st.N) nseg *= 2;
+    while (nseg < 16 && (npix + 31) / 32 * nseg < 4 * 148 && 2 * nseg * (long long)st.M <= st.N) nseg *= 2;
     return nseg;
 }
 
@@ -912,6 +939,27 @@ int check_device_flag(ks_context* c, const char* what) {
     return KS_OK;
 }
 
+// The thin image from the splat table `tab` into `out` (through `perm` if given); `resid`: with the anchor residuals.
+// Allocates nothing: the pieces' sums have their place since regenerate.
+template <class T>
+int launch_thin(ks_context* c, const double* tab, int nsplat, double t_obs, const long long* perm, double* out, bool resid) {
+    const int nseg = thin_pieces(c->st, c->npix);
+    const size_t smem = (sizeof(MarchShared<T>) + 15) / 16 * 16 + size_t(nsplat) * kThinRow * sizeof(T);
+    double* rt = resid ? c->resid_t.as<double>() : nullptr;
+    double* rp = resid ? c->resid_phi.as<double>() : nullptr;
+    KS_CUDA(c, cudaFuncSetAttribute(k_thin<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    k_thin<T><<<dim3(nblocks(c->npix, 32), nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, c->npix, tab, nsplat, t_obs, nseg,
+                                                                            c->thin_part.as<double>(), perm, out, rt, rp);
+    c->launches++;
+    KS_CUDA(c, cudaGetLastError());
+    if (nseg > 1) {
+        k_thin_sum<<<nblocks(c->npix), kBlock, 0, c->stream>>>(c->npix, nseg, c->thin_part.as<double>(), perm, out, rt, rp);
+        c->launches++;
+        KS_CUDA(c, cudaGetLastError());
+    }
+    return KS_OK;
+}
+
 // Write `nvec` x npix x width doubles from the sorted device buffer to `out` (host or device) in `order`.
 int emit(ks_context* c, const double* sorted, int width, int nvec, int order, double* out) {
     size_t bytes = size_t(c->npix) * width * nvec * sizeof(double);
@@ -1164,6 +1212,7 @@ int regenerate_impl(ks_context* c, double a, double theta_o, int32_t nsamples, i
     c->launches++;
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, c->resid_t.ensure(n * sizeof(double)));
+    if (thin_pieces(st, n) > 1) KS_CUDA(c, c->thin_part.ensure(3 * size_t(thin_pieces(st, n)) * n * sizeof(double)));
     KS_CUDA(c, c->resid_phi.ensure(n * sizeof(double)));
     KS_CUDA(c, cudaMemsetAsync(c->resid_t.p, 0, n * sizeof(double), c->stream));
     KS_CUDA(c, cudaMemsetAsync(c->resid_phi.p, 0, n * sizeof(double), c->stream));
@@ -1258,22 +1307,13 @@ int ks_thin_image(ks_context* c, const double* params, int32_t nsplat, double t_
         KS_CUDA(c, cudaGetLastError());
     }
     KS_CUDA(c, c->out_sorted.ensure(n * sizeof(double)));
-    size_t smem = size_t(nsplat) * ST_COUNT * (precision == KS_FP64 ? sizeof(double) : sizeof(float));
-    if (smem > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", nsplat);
-    const int nseg = thin_pieces(c->st);
+    if (size_t(nsplat) * ST_COUNT * (precision == KS_FP64 ? sizeof(double) : sizeof(float)) > 200 * 1024)
+        return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", nsplat);
     cudaEventRecord(c->ev0, c->stream);
-    if (precision == KS_FP64) {
-        KS_CUDA(c, cudaFuncSetAttribute(k_thin<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<double><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nseg, nullptr,
-                                                                 c->out_sorted.as<double>(), c->resid_t.as<double>(), c->resid_phi.as<double>());
-    } else {
-        KS_CUDA(c, cudaFuncSetAttribute(k_thin<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<float><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, c->tab.as<double>(), nsplat, t_obs, nseg, nullptr,
-                                                                c->out_sorted.as<double>(), nullptr, nullptr);
-    }
+    int sl = precision == KS_FP64 ? launch_thin<double>(c, c->tab.as<double>(), nsplat, t_obs, nullptr, c->out_sorted.as<double>(), true)
+                                  : launch_thin<float>(c, c->tab.as<double>(), nsplat, t_obs, nullptr, c->out_sorted.as<double>(), false);
+    if (sl) return sl;
     cudaEventRecord(c->ev1, c->stream);
-    c->launches++;
-    KS_CUDA(c, cudaGetLastError());
     int s = emit(c, c->out_sorted.as<double>(), 1, 1, order, out);
     if (s) return s;
     KS_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -2515,17 +2555,8 @@ int ks_thin_image_noalloc(ks_context* c, const double* params, int32_t nsplat, d
         KS_CUDA(c, cudaGetLastError());
     }
     const long long* perm = order == KS_ORDER_SCREEN ? c->perm.as<long long>() : nullptr;
-    const size_t smem = size_t(nsplat) * ST_COUNT * (precision == KS_FP64 ? sizeof(double) : sizeof(float));
-    const int nseg = thin_pieces(c->st);
-    if (precision == KS_FP64) {
-        KS_CUDA(c, cudaFuncSetAttribute(k_thin<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<double><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, nseg, perm, out, nullptr, nullptr);
-    } else {
-        KS_CUDA(c, cudaFuncSetAttribute(k_thin<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_thin<float><<<nblocks(n, kBlock / nseg), kBlock, smem, c->stream>>>(plan_view(c), c->st, n, tab, nsplat, t_obs, nseg, perm, out, nullptr, nullptr);
-    }
-    c->launches++;
-    KS_CUDA(c, cudaGetLastError());
+    int sl = precision == KS_FP64 ? launch_thin<double>(c, tab, nsplat, t_obs, perm, out, false) : launch_thin<float>(c, tab, nsplat, t_obs, perm, out, false);
+    if (sl) return sl;
     KS_CUDA(c, cudaStreamSynchronize(c->stream));
     return KS_OK;
 }

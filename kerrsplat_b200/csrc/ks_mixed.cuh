@@ -4,6 +4,7 @@
 // k_stream marches every ray once (the recurrence and the quadrature, re-anchored to the FP64 table every M
 // samples) into a sample stream that every frame, frequency and parameter set reads.
 #pragma once
+#include "ks_march_block.cuh"
 #include "ks_transfer.cuh"
 
 namespace ks {
@@ -186,6 +187,29 @@ __global__ void __launch_bounds__(128, 4) k_stream(PlanView P, Spacetime st, lon
         atomicMax(&resid_phi[j0 + j], (unsigned long long)__double_as_longlong(rp));
     } else {
         march_range(P, j0 + j, R, sink, k0, k1);
+    }
+}
+
+// A block per (32 rays, segment of seg_len samples starting at an anchor multiple) of the rays [j0, j0 + npix), the
+// samples by march_block. The FP64 stream also leaves the anchor residuals of its rays (the largest over the segments).
+template <class T, class S>
+__global__ void __launch_bounds__(32 * kMarchWarps, sizeof(T) == 4 ? 4 : 3)
+k_stream_block(PlanView P, Spacetime st, long long j0, long long npix, long long npad, int seg_len, S* __restrict__ out,
+               unsigned long long* __restrict__ resid_t, unsigned long long* __restrict__ resid_phi) {
+    extern __shared__ __align__(16) unsigned char march_smem[];
+    MarchShared<T>& shared = *reinterpret_cast<MarchShared<T>*>(march_smem);
+    const int lane = threadIdx.x & 31;
+    const bool live = blockIdx.x * 32LL + lane < npix;
+    const long long j = live ? blockIdx.x * 32LL + lane : npix - 1;
+    const int k0 = 1 + blockIdx.y * seg_len, k1 = min(st.N + 1, k0 + seg_len);
+    const double temp = sqrt(1.0 - st.a * st.a);
+    StreamSink<T, S> sink{out, npad, j, T(st.a), T(st.rh * (1 + 1e-3)), T(1.0 + temp), T(1.0 - temp), float(st.a / (2.0 * temp))};
+    double rt, rp;
+    march_block<sizeof(S) == 8>(P, st, j0 + j, live, k0, k1, shared, sink, rt, rp);
+    if (sizeof(S) == 8 && threadIdx.x < 32 && live) {
+        // non-negative doubles order as integers
+        atomicMax(&resid_t[j0 + j], (unsigned long long)__double_as_longlong(rt));
+        atomicMax(&resid_phi[j0 + j], (unsigned long long)__double_as_longlong(rp));
     }
 }
 

@@ -17,6 +17,10 @@
 // is linear in a splat's constants (the centre, the quaternion, the field's angles) is left as sums over samples
 // and turned into parameter rows once, in FP64. Each splat's sums of a window are formed by one warp in a fixed
 // order and every unit has its own block of partial sums, so the gradient is the same bit for bit.
+//
+// Bound by instruction issue (41% of the issue slots at 12 warps per SM, its registers' limit). 224 x 224 x 896, 64 splats,
+// two frequencies: 10.6 ms; the step and element kernels before it took 28.7 ms. Four blocks per SM (128 registers) spill:
+// the whole gradient 23.6 ms against 22.5.
 #pragma once
 #include "ks_gradient.cuh"
 #include "ks_transport.cuh"
@@ -243,7 +247,7 @@ __device__ __forceinline__ void pair_adjoint(const T* r, T x, T y, T z, T t, con
                                              const T* cbs, T* v) {
     const T dt = t - r[RW_T0];
     T sp, cp;
-    fsincos(r[RW_OMEGA] * dt, sp, cp);
+    sincos_product(r[RW_OMEGA], dt, sp, cp);
     const T cx = r[RW_CX], cy = r[RW_CY];
     const T d0 = x - (cx * cp - cy * sp), d1 = y - (cx * sp + cy * cp);
     const T dr[3] = {d0 * cp + d1 * sp, -d0 * sp + d1 * cp, z - r[RW_CZ]};
@@ -251,7 +255,7 @@ __device__ __forceinline__ void pair_adjoint(const T* r, T x, T y, T z, T t, con
 #pragma unroll
     for (int j = 0; j < 3; ++j) e[j] = r[RW_A0 + j] * dr[0] + r[RW_A3 + j] * dr[1] + r[RW_A6 + j] * dr[2];
     const T tt = dt * r[RW_INVW];
-    const T ne = r[RW_NE] * hexp(-(e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + tt * tt) * T(0.5));
+    const T ne = r[RW_NE] * weight_of((e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + tt * tt) * T(0.5));
     const LFrame<T> lf = row_frame(F, r, alpha, beta, a_sin_tho);
     T sb, cb;
     pitch_sc(lf.cosB, sb, cb);
@@ -457,7 +461,7 @@ k_reverse(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ rows
                         const T dr = rho - r[RW_RHO], dz = z - r[RW_CZ];
                         if (dr * dr + dz * dz > r[RW_SUPP]) continue;
                         T q;
-                        if (!row_exponent(r, t, x, yy, z, true, q)) continue;
+                        if (!row_exponent<true>(r, t, x, yy, z, q)) continue;
                         if (q < T(kQCUT)) m |= 1u << b;
                     }
                     masks[(kl * nw + wd) * 32 + lane] = m;

@@ -124,15 +124,43 @@ __device__ __forceinline__ double hln(double x) { return log(x); }
 
 // ---- the pair arithmetic ---------------------------------------------------------------------------------
 
-// The weight exponent of a splat row at (t, x, y, z); `cull` as splat_exponent.
-template <class T>
-__device__ __forceinline__ bool row_exponent(const T* r, T t, T x, T y, T z, bool cull, T& q) {
+// Sine and cosine of the product a b, to FP32's rounding: the product's own rounding error is carried, the reduction
+// by pi/2 is in two parts (Cody & Waite 1980) and the series run on [-pi/4, pi/4]. The hardware pair is good to 4e-7,
+// which moves a centre at 10 M by 4e-6 M and the weight of a splat 0.3 M wide by some 1e-5: the largest error of an
+// evaluation. A test needs no better than that (its cutoff is a weight of 1e-6).
+__device__ __forceinline__ void sincos_product(float a, float b, float& s, float& c) {
+    const float p = a * b, lo = fmaf(a, b, -p);
+    const float k = rintf(p * 0.63661977236758134f);
+    float x = fmaf(-k, 1.57079637050628662f, p);
+    x += fmaf(-k, -4.37113900018624283e-8f, lo);
+    const float x2 = x * x;
+    const float sn = fmaf(x * x2, fmaf(x2, fmaf(x2, fmaf(x2, 1.f / 362880.f, -1.f / 5040.f), 1.f / 120.f), -1.f / 6.f), x);
+    const float cs = fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 1.f / 40320.f, -1.f / 720.f), 1.f / 24.f), -0.5f), 1.f);
+    const int q = int(k);
+    s = (q & 1) ? cs : sn;
+    c = (q & 1) ? sn : cs;
+    if (q & 2) s = -s;
+    if ((q + 1) & 2) c = -c;
+}
+__device__ __forceinline__ void sincos_product(double a, double b, double& s, double& c) { fsincos(a * b, s, c); }
+// exp(-q), the rounding of q log2(e) carried
+__device__ __forceinline__ float weight_of(float q) {
+    const float y = q * -1.4426950408889634f, lo = fmaf(q, -1.4426950408889634f, -y) - q * 1.9259629e-8f;
+    const float e = hexp2(y);
+    return fmaf(e, lo * 0.6931471805599453f, e);
+}
+__device__ __forceinline__ double weight_of(double q) { return exp(-q); }
+
+// The weight exponent of a splat row at (t, x, y, z). TEST: as a test needs it, with splat_exponent's cull.
+template <bool TEST, class T>
+__device__ __forceinline__ bool row_exponent(const T* r, T t, T x, T y, T z, T& q) {
     const T dt = t - r[RW_T0];
     T sp, cp;
-    fsincos(r[RW_OMEGA] * dt, sp, cp);
+    if constexpr (TEST) fsincos(r[RW_OMEGA] * dt, sp, cp);
+    else sincos_product(r[RW_OMEGA], dt, sp, cp);
     const T cx = r[RW_CX] * cp - r[RW_CY] * sp, cy = r[RW_CX] * sp + r[RW_CY] * cp;
     const T d0 = x - cx, d1 = y - cy, d2 = z - r[RW_CZ];
-    if (cull && d0 * d0 + d1 * d1 + d2 * d2 > r[RW_SUPP]) return false;
+    if (TEST && d0 * d0 + d1 * d1 + d2 * d2 > r[RW_SUPP]) return false;
     const T a = d0 * cp + d1 * sp, b = -d0 * sp + d1 * cp;
     const T e0 = r[RW_A0] * a + r[RW_A3] * b + r[RW_A6] * d2;
     const T e1 = r[RW_A1] * a + r[RW_A4] * b + r[RW_A7] * d2;
@@ -670,7 +698,7 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                                 // farther from the circle the centre runs on than the support: outside at every time
                                 const T dr = rho - r[RW_RHO], dz = z - r[RW_CZ];
                                 if (dr * dr + dz * dz > r[RW_SUPP]) continue;
-                                if (!row_exponent(r, t, x, yy, z, true, q)) continue;
+                                if (!row_exponent<true>(r, t, x, yy, z, q)) continue;
                             } else {
                                 const T dx = x - r[RW_CX], dy = yy - r[RW_CY], dz = z - r[RW_CZ];
                                 if (dx * dx + dy * dy + dz * dz > r[RW_RHO]) continue;   // outside the knots' bounding sphere
@@ -754,9 +782,9 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                                 m &= m - 1;
                                 const T* sr = rows + (long long)(wd * 32 + b) * ST;
                                 T q;
-                                if (KM == 1 || int(sr[RW_KIND]) != KS_KNOT21) row_exponent(sr, t, x, yy, z, false, q);
+                                if (KM == 1 || int(sr[RW_KIND]) != KS_KNOT21) row_exponent<false>(sr, t, x, yy, z, q);
                                 else row_knot_exponent(sr, knots, t, x, yy, z, q);
-                                const T ne = sr[RW_NE] * fexp(-q);
+                                const T ne = sr[RW_NE] * weight_of(q);
                                 const LFrame<T> lf = row_frame(F, sr, alpha, beta, a_sin_tho);
                                 T sb, cb;
                                 pitch_sc(lf.cosB, sb, cb);
@@ -803,8 +831,9 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                     ev[6]++;
                     if (gstate) {
                         const int at = order2[id];
-                        const long long combo = (long long)(v0 + c) * job.nframes + f;
-                        put16<12>(gstate + ((combo * N + (kr + (at >> 5) - 1)) * npad + jb + (at & 31)) * 32 + 16, v);
+                        const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + (at >> 5) - 1)) * npad + jb + (at & 31);
+                        put16<12>(gstate + g * 32 + 16, v);
+                        job.gact[g] = 1;
                     }
                     T w[kRec];
                     step_record(c_moments, v, v[11], w);
@@ -826,7 +855,6 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                         if (gstate) {
                             const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + kl - 1)) * npad + jb + lane;
                             put16<4>(gstate + g * 32 + 4 * row, pr[q]);
-                            if (row == 0) job.gact[g] = 1;
                         }
                         T p1[4], p2[4], p3[4];
                         kvec_t(v + 8, pr[q], p1); kvec_t(v + 8, p1, p2); kvec_t(v + 8, p2, p3);
