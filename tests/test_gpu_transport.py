@@ -70,6 +70,20 @@ def test_transport_edges(oracle, na, nb, N, ns, nf, nmax):
     cache.close()
 
 
+@pytest.mark.parametrize("shift", [-12.0, -4.0, 0.0, 2.0])
+def test_step_adjoint_strengths(shift):
+    """The FP32 step adjoint on weak steps (its power series) and strong ones (its FP64 partials): electron densities
+    e^shift apart put the squared strength of a step below, across and above 1/8."""
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), (17, 15))
+    cache, p = cache_of(cam, 96), wide_splats(12, 8)
+    p[12] += shift
+    nus, m = [86e9, 230e9], ks.PolarizedSplats(p)
+    ds = np.random.Generator(np.random.PCG64(9)).standard_normal(np.shape(ks.render(cache, m, [2.0], nus, L)))
+    g64 = ks.adjoint(cache, m, [2.0], nus, L, ds)
+    assert rel(ks.adjoint(cache, m, [2.0], nus, L, ds, precision=ks.KS_MIXED), g64) < 1e-3
+    cache.close()
+
+
 @pytest.mark.parametrize("N,uneven", [(1, None), (63, None), (65, None), (129, None), (1000, None), (640, (300.0, 64))])
 def test_thin_pieces(oracle, N, uneven):
     cam = ks.Camera((-11.9, 12.3), (-12.1, 11.7), (13, 11))
