@@ -36,18 +36,83 @@ enum RowField {
     RW_A0, RW_A1, RW_A2, RW_A3, RW_A4, RW_A5, RW_A6, RW_A7, RW_A8, RW_U1, RW_U2, RW_U3,
     RW_BX, RW_BY, RW_BZ, RW_GQ, RW_GAM, RW_TE, RW_F0, RW_KR, RW_NUC, RW_SUPP, RW_KIND, RW_ANG,
     RW_THERMAL_COUNT,
-    // power law and kappa constants, the field strength their fits take, and the knot record
     RW_DF0 = RW_THERMAL_COUNT, RW_DKR,   // thermal tables with a gradient: the Bessel ratios' derivatives by ln Te
-    RW_E0 = RW_THERMAL_COUNT, RW_E1, RW_E2, RW_E3, RW_E4, RW_E5, RW_E6, RW_E7, RW_E8, RW_BMAG, RW_KOFF, RW_NK,
-    RW_COUNT
+    // scenes of several populations: the knot record, then the constants of the power-law and kappa fits
+    // (population_constants)
+    RW_KOFF = RW_THERMAL_COUNT, RW_NK, RW_E, RW_ECOUNT = 32, RW_COUNT = RW_E + RW_ECOUNT
 };
 template <class T, int KM>
 __host__ __device__ constexpr int row_stride() {
-    return KM == 1 ? (sizeof(T) == 4 ? 36 : 34) : (sizeof(T) == 4 ? 44 : 46);
+    return KM == 1 ? (sizeof(T) == 4 ? 36 : 34) : (sizeof(T) == 4 ? 68 : 66);
 }
-static_assert(RW_THERMAL_COUNT <= 34 && RW_COUNT <= 44, "rows hold their fields");
+static_assert(RW_DKR < 34 && RW_COUNT <= 66, "rows hold their fields");
 
 constexpr double kNUC = kEE / (2.0 * 3.141592653589793 * kME * kCL);   // cyclotron frequency per gauss
+
+// the logarithm of the base that hlog2 and hexp2 pair on: 2 in FP32, e in FP64
+template <class T> __device__ __forceinline__ double row_log(double v) { return sizeof(T) == 4 ? log2(v) : log(v); }
+
+// What the power-law fits (powerlaw_cs) and the kappa fits (kappa_cs) take from the splat alone, formed once in FP64:
+// some twenty powers an evaluation otherwise. 112 x 112 rays x up to 2048 samples, 96 splats of three populations, four
+// frequencies, two frames: k_transport 17.0 -> 12.1 ms. The wider rows (68 words against 44 in FP32) stay in global
+// memory for tables that shared memory does not hold.
+enum PowerField { EP_J, EP_JQ, EP_JV, EP_A, EP_AQ, EP_AV, EP_RQ, EP_RV, EP_P1, EP_PH, EP_PG };
+enum KappaField {
+    EK_X,                                                    // 1 / (w kappa)^2
+    EK_I = 1, EK_Q = 5, EK_AI = 9, EK_AQ = 13,               // a bridge each: low limit, x slope, x ln(low / high), 1 / x
+    EK_V = 17, EK_AV = 22,                                   // low, slope, ln(low / high), x, 1 / x without the pitch angle's part
+    EK_FIT = 27, EK_FQ0, EK_FQ1, EK_FV0, EK_FV1 = 31         // rotativity fits: the lower one's index, the four amplitudes
+};
+template <class T>
+__device__ void population_constants(const double* p, T* e) {
+    constexpr double PI = 3.141592653589793;
+    const double ej = kEE * kEE / kCL, ea = kEE * kEE / (kME * kCL);
+    if (int(p[ST_KIND]) == KS_POWERLAW22) {
+        const double q = p[ST_P], gm = p[ST_GMIN], sp = p[ST_GSPAN];
+        e[EP_J] = T(ej * pow(3.0, q / 2) * (q - 1) / (2 * (q + 1) * sp) * p[ST_GAMJ]);
+        e[EP_JQ] = T((q + 1) / (q + 7.0 / 3));
+        e[EP_JV] = T(171.0 / 250 * pow(q, 49.0 / 100) * sqrt(3.0));
+        e[EP_A] = T(ea * pow(3.0, (q + 1) / 2) * (q - 1) / (4 * sp) * p[ST_GAMA]);
+        e[EP_AQ] = T(pow(17.0 / 500 * q - 43.0 / 1250, 43.0 / 500));
+        e[EP_AV] = T(pow(71.0 / 100 * q + 22.0 / 625, 197.0 / 500));
+        e[EP_RQ] = T(-ea * (q - 1) / sp * pow(gm, 2 - q) / (q / 2 - 1));
+        e[EP_RV] = T(2 * (q + 2) / (q + 1) * ea * (q - 1) / sp * pow(gm, -(q + 1)) * log(gm));
+        e[EP_P1] = T((q - 1) / 2);
+        e[EP_PH] = T(q / 2 - 1);
+        e[EP_PG] = T((q / 2 - 1) * row_log<T>(gm * gm));
+    } else if (int(p[ST_KIND]) == KS_KAPPA22) {
+        const double k = p[ST_KAP], w = p[ST_W], sj = (3 * k - 4) / 6, sa = (3 * k - 1) / 6;
+        auto bridge = [&](int f, double scale, double lo, double hi, double xx, double slope) {
+            e[f] = T(scale * lo); e[f + 1] = T(xx * slope); e[f + 2] = T(xx * row_log<T>(lo / hi)); e[f + 3] = T(1 / xx);
+        };
+        auto bridge_v = [&](int f, double scale, double lo, double hi, double xx, double slope) {
+            e[f] = T(scale * lo); e[f + 1] = T(slope); e[f + 2] = T(row_log<T>(lo / hi)); e[f + 3] = T(xx); e[f + 4] = T(1 / xx);
+        };
+        e[EK_X] = T(1 / ((w * k) * (w * k)));
+        const double g = 4 * PI * p[ST_G43] / (12.980246132766677 * p[ST_G2]), hk = 0.25 * pow(3.0, (k - 1) / 2) * (k - 2) * (k - 1) * p[ST_GQ] * p[ST_GP];
+        bridge(EK_I, ej, g, hk, 3 * pow(k, -1.5), sj);
+        bridge(EK_Q, ej, 0.5 * g, (0.64 + k / 50) * hk, 3.7 * pow(k, -1.6), sj);
+        bridge_v(EK_V, ej, 0.5625 * pow(k, -66.0 / 125) / w * g, 0.765625 * pow(k, -11.0 / 25) / w * hk, 3 * pow(k, -1.5), sj);
+        const double ck = (k - 2) * (k - 1) * k;
+        const double base = 1.2009369551760027 * (10.0 / 41) * 4 * PI * PI / pow(w * k, 16.0 / 3 - k) * ck / (3 * k - 1) * 0.9027452929509336 * p[ST_HYP];
+        const double hi = 2 * pow(PI, 2.5) / 3 * ck / pow(w * k, 5.0) * (2 * p[ST_GK2] / (2 + k) - 1);
+        const double es = kEE * kNUC;   // n_e e / (B sin theta_B) = n_e es / (nu_c sin theta_B)
+        bridge(EK_AI, es, base, hi * (pow(3 / k, 19.0 / 4) + 3.0 / 5), pow(-7.0 / 4 + 8 * k / 5, -43.0 / 50), sa);
+        bridge(EK_AQ, es, 25.0 / 48 * base, (441 * pow(k, -144.0 / 25) + 11.0 / 20) * hi, 1.4 * pow(k, -23.0 / 20), sa);
+        bridge_v(EK_AV, es, 77 / (100 * w) * pow(k, -0.7) * base,
+                 14.3 * pow(w, -116.0 / 125) * (169 * pow(k, -8.0) + 13.0 / 2500 * k - 263.0 / 5000 + 47 / (200 * k)) * hi,
+                 1.22 * pow(k, -142.0 / 125) + 7.0 / 1000, sa);
+        const double kc = fmin(5.0, fmax(3.5, k)), s = sqrt(w), x = s * exp(-5 * w);
+        const int i = kc < 4.0 ? 0 : kc < 4.5 ? 1 : 2;
+        const double f = (kc - 3.5 - 0.5 * i) * 2;
+        const double q[4] = {17 * w - 3 * s + 7 * x, 46 * w / 3 - 5 * s / 3 + 17 * x / 3, 14 * w - 13 * s / 8 + 9 * x / 2, 25 * w / 2 - s + 5 * x};
+        const double v[4] = {(w * w + 2 * w + 1) / (25 * w * w / 8 + 4 * w + 1), (w * w + 54 * w + 50) / (30 * w * w / 11 + 134 * w + 50),
+                             (w * w + 43 * w + 38) / (7 * w * w / 3 + 185 * w / 2 + 38), (w + 13.0 / 14) / (2 * w + 13.0 / 14)};
+        e[EK_FIT] = T(i);
+        e[EK_FQ0] = T(-ea * (1 - f) * q[i]); e[EK_FQ1] = T(-ea * f * q[i + 1]);
+        e[EK_FV0] = T(2 * ea * p[ST_KB] * (1 - f) * v[i]); e[EK_FV1] = T(2 * ea * p[ST_KB] * f * v[i + 1]);
+    }
+}
 
 // rows of the concatenated FP64 table, then the knot array; `total` values, the tail zero
 template <class T, int KM>
@@ -90,17 +155,18 @@ __global__ void k_rows(int ntot, int nkv, long long total, const double* __restr
     if (f >= RW_A0 && f <= RW_A8) v = p[ST_R0 + (f - RW_A0)] * p[ST_ES1 + (f - RW_A0) % 3];
     if (KM == 1 && gtab && f == RW_DF0) v = gtab[(q / ST) * GT_COUNT + GT_DF0];
     if (KM == 1 && gtab && f == RW_DKR) v = gtab[(q / ST) * GT_COUNT + GT_DKR];
-    if (KM != 1 && f >= RW_E0 && f < RW_COUNT) {
-        const int e = f - RW_E0;
-        if (f == RW_BMAG) v = p[ST_BMAG];
-        else if (f == RW_KOFF) v = p[ST_KOFF];
+    if (KM != 1) {
+        if (f == RW_KOFF) v = p[ST_KOFF];
         else if (f == RW_NK) v = p[ST_NK];
-        else if (int(p[ST_KIND]) == KS_POWERLAW22) v = e == 0 ? p[ST_P] : e == 1 ? p[ST_GMIN] : e == 2 ? p[ST_GSPAN] : e == 3 ? p[ST_GAMJ] : e == 4 ? p[ST_GAMA] : 0.0;
-        else if (int(p[ST_KIND]) == KS_KAPPA22) v = p[ST_KAP + e];   // kappa, w, hyp, the five gammas, kb
+        else if (f == RW_E) {   // one thread forms a splat's population constants
+            for (int k = 0; k < RW_ECOUNT; ++k) out[q + k] = T(0);
+            population_constants(p, out + q);
+            return;
+        } else if (f > RW_E && f < RW_COUNT) return;
     }
     out[q] = T(v);
 }
-static_assert(ST_KB - ST_KAP == 8, "the kappa constants are nine consecutive table fields");
+static_assert(EK_FV1 < RW_ECOUNT, "rows hold the kappa constants");
 
 // ---- hardware functions -----------------------------------------------------------------------------------
 // The FP32 forms are one instruction each: the approximations that -prec-div=false and the __-functions compile
@@ -273,17 +339,70 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     return jI > T(0) || c[6] != T(0) || c[7] != T(0);
 }
 
-// The other populations' fits, out of line: scenes that mix populations run them a population at a time.
+// The power-law and kappa fits (powerlaw_cs, kappa_cs) from the row's constants, out of line: scenes that mix
+// populations run them a population at a time. As there, a field along the ray is evaluated 1e-6 from the axis.
+template <class T>
+__device__ __forceinline__ T kappa_bridge(T lo, T arg, T ix) { return lo * hexp2(-ix * hlog2(T(1) + hexp2(arg))); }
+
 template <class T>
 __device__ __noinline__ bool other_row(const T* r, int kind, T ne, T nu, T st, T ct, T* c) {
-    Coef<T> f;
-    if (kind == KS_POWERLAW22)
-        f = powerlaw_cs(ne, r[RW_E0], r[RW_E1], r[RW_E2], r[RW_E3], r[RW_E4], r[RW_BMAG], nu, st, ct);
-    else
-        f = kappa_cs(ne, r[RW_E0], r[RW_E1], r[RW_E2], r[RW_E3], r[RW_E4], r[RW_E5], r[RW_E6], r[RW_E7], r[RW_E8], r[RW_BMAG], nu, st, ct);
-    const T fe = row_cap(f.jI, f.jQ, f.jV), fa = row_cap(f.aI, f.aQ, f.aV);
-    c[0] = f.jI; c[1] = f.jQ * fe; c[2] = f.jV * fe; c[3] = f.aI; c[4] = f.aQ * fa; c[5] = f.aV * fa; c[6] = f.rQ; c[7] = f.rV;
-    return f.jI > T(0) || f.aI > T(0) || f.rQ != T(0) || f.rV != T(0);
+    st = fmax(st, T(1e-6));
+    const T* e = r + RW_E;
+    const T nc = r[RW_NUC], nb = nc * st, inu = hrcp(nu), ist = hrcp(st), ls = hlog2(st);
+    const T sg = ct > T(0) ? T(1) : (ct < T(0) ? T(-1) : T(0));
+    T jI, jQ, jV, aI, aQ, aV, rQ, rV;
+    if (kind == KS_POWERLAW22) {
+        const T xx = nu * hrcp(nb), lx = hlog2(xx), ix = hrsqrt(xx);
+        const T pw = hexp2(-e[EP_P1] * lx);                      // xx^(-(p - 1) / 2)
+        jI = ne * nb * e[EP_J] * pw;
+        jQ = e[EP_JQ] * jI;
+        jV = e[EP_JV] * ct * ist * ix * jI;
+        aI = ne * inu * e[EP_A] * pw * ix * ix * ix;             // xx^(-(p + 2) / 2)
+        aQ = e[EP_AQ] * aI;
+        const T t6 = T(31.0 / 10) * hexp2(T(-48.0 / 25) * ls) - T(31.0 / 10);
+        aV = t6 > T(0) ? e[EP_AV] * hexp2(T(64.0 / 125) * hlog2(t6)) * ix * sg * aI : T(0);
+        rQ = ne * e[EP_RQ] * (nb * inu) * (nb * inu) * inu * (T(1) - hexp2(e[EP_PG] - e[EP_PH] * lx));
+        rV = ne * e[EP_RV] * nb * inu * inu * ct * ist;
+    } else {
+        const T X = nu * hrcp(nb) * e[EK_X], lx = hlog2(X);
+        const T pj = ne * nb * hexp2(T(1.0 / 3) * lx), pa = ne * hrcp(nb) * hexp2(T(-5.0 / 3) * lx);
+        jI = pj * kappa_bridge(e[EK_I], e[EK_I + 1] * lx + e[EK_I + 2], e[EK_I + 3]);
+        jQ = pj * kappa_bridge(e[EK_Q], e[EK_Q + 1] * lx + e[EK_Q + 2], e[EK_Q + 3]);
+        aI = pa * kappa_bridge(e[EK_AI], e[EK_AI + 1] * lx + e[EK_AI + 2], e[EK_AI + 3]);
+        aQ = pa * kappa_bridge(e[EK_AQ], e[EK_AQ + 1] * lx + e[EK_AQ + 2], e[EK_AQ + 3]);
+        // circular: the limits carry (sin^-u - 1)^v and X^-0.35 against X^-0.5
+        const T u1 = hexp2(T(-12.0 / 5) * ls) - T(1), u2 = hexp2(T(-2.5) * ls) - T(1);
+        const T u3 = hexp2(T(-114.0 / 50) * ls) - T(1), u4 = hexp2(T(-41.0 / 20) * ls) - T(1);
+        const T x35 = hexp2(T(-7.0 / 20) * lx);
+        jV = aV = T(0);
+        if (u1 > T(0) && u2 > T(0)) {
+            const T l1 = T(12.0 / 25) * hlog2(u1), l2 = T(11.0 / 25) * hlog2(u2);
+            jV = sg * pj * x35 * kappa_bridge(e[EK_V] * hexp2(l1), e[EK_V + 3] * (e[EK_V + 1] * lx + e[EK_V + 2] + l1 - l2 + T(3.0 / 20) * lx), e[EK_V + 4]);
+        }
+        if (u3 > T(0) && u4 > T(0)) {
+            const T l3 = T(223.0 / 500) * hlog2(u3), l4 = T(0.5) * hlog2(u4);
+            aV = sg * pa * x35 * kappa_bridge(e[EK_AV] * hexp2(l3), e[EK_AV + 3] * (e[EK_AV + 1] * lx + e[EK_AV + 2] + l3 - l4 + T(3.0 / 20) * lx), e[EK_AV + 4]);
+        }
+        const int i = int(e[EK_FIT]);
+        auto fit_q = [&](int n) {
+            const T k84 = n == 0 ? T(1.0 / 30) : n == 1 ? T(1.0 / 18) : n == 2 ? T(1.0 / 12) : T(1.0 / 8);
+            const T ks_ = n == 0 ? T(1.0 / 10) : n == 1 ? T(1.0 / 6) : n == 2 ? T(1.0 / 4) : T(3.0 / 8);
+            const T kx = n == 0 ? T(1.5) : n == 1 ? T(1.75) : n == 2 ? T(2) : T(2.25);
+            const T kp = n == 0 ? T(0.471) : n == 1 ? T(0.5) : n == 2 ? T(0.525) : T(0.541);
+            T s, cs;
+            sincos_product(fmin(X, T(1e6)), ks_, s, cs);   // beyond, its factor has vanished
+            return T(1) - hexp(-k84 * hexp2(T(0.84) * lx)) - s * hexp(-kx * hexp2(kp * lx));
+        };
+        auto fit_v = [&](int n) {
+            const T k = n == 0 ? T(0.447) : n == 1 ? T(0.391) : n == 2 ? T(0.348) : T(0.313);
+            return T(1) - T(0.17) * hln(T(1) + k * hexp2(T(-0.5) * lx));
+        };
+        rQ = ne * (nb * inu) * (nb * inu) * inu * (e[EK_FQ0] * fit_q(i) + e[EK_FQ1] * fit_q(i + 1));
+        rV = ne * nc * ct * inu * inu * (e[EK_FV0] * fit_v(i) + e[EK_FV1] * fit_v(i + 1));
+    }
+    const T fe = row_cap(jI, jQ, jV), fa = row_cap(aI, aQ, aV);
+    c[0] = jI; c[1] = jQ * fe; c[2] = jV * fe; c[3] = aI; c[4] = aQ * fa; c[5] = aV * fa; c[6] = rQ; c[7] = rV;
+    return jI > T(0) || aI > T(0) || rQ != T(0) || rV != T(0);
 }
 
 // 2^floor(log2 v) of a normal positive v (the exponent alone), 1 otherwise

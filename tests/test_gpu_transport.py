@@ -116,6 +116,43 @@ def test_tables_past_shared_memory(oracle):
     cache.close()
 
 
+@pytest.mark.parametrize("nf", [1, 4])
+def test_population_fits(oracle, nf):
+    """Power-law and kappa fits from their splats' constants: indices around 2 and in each interval of the kappa
+    rotativity fits, the intervals' ends and beyond them, narrow and wide kappa distributions."""
+    rng = np.random.Generator(np.random.PCG64(12))
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), (9, 7))
+    cache = cache_of(cam, 70)
+    pp, pk = scenes.powerlaw_params(rng, 4, A), scenes.kappa_params(rng, 9, A)
+    for q in (pp, pk):
+        q[3:6] = np.log(rng.uniform(0.8, 2.0, q[3:6].shape))
+    pp[13] = [1.9, 2.1, 2.5, 3.5]
+    pk[13] = [3.05, 3.5, 3.75, 4.0, 4.25, 4.5, 4.75, 5.0, 6.5]
+    pk[14] = np.log([0.3, 1.0, 3.0, 50.0, 20.0, 10.0, 5.0, 2.0, 1.0])
+    kap = ks.KappaSplats(pk)
+    m, nus = ks.CompositeModel(ks.PowerLawSplats(pp), kap), np.geomspace(43e9, 690e9, 4)[:nf]
+    plain = np.asarray(ks.render(cache, m, [3.0], nus, L))
+    for v in range(nf):
+        ref = oracle.polarized_image(A, THO, cam.alpha, cam.beta, 70, 64, [("powerlaw", pp, None), ("kappa", pk, kap.hyp)], 3.0, nus[v], L)
+        assert rel(plain[v, 0], ref) < 1e-9, v
+    assert rel(np.asarray(ks.render(cache, m, [3.0], nus, L, precision=ks.KS_MIXED)), plain) < 1e-4
+    cache.close()
+
+
+def test_fp32_rows_in_global_memory(oracle):
+    # 500 knot splats with ten knots each: within the largest FP32 table, past a block's shared memory with its rows
+    p = wide_splats(500, 13)
+    p[3:6] -= 1.5
+    times = np.linspace(-60.0, 40.0, 10)
+    knots = scenes.trajectory_knots(p, A, times)
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), (9, 7))
+    cache = cache_of(cam, 40)
+    ref = oracle.polarized_image(A, THO, cam.alpha, cam.beta, 40, 64, [("knot", p, None, knots, times)], 3.0, 230e9, L)
+    img = np.asarray(ks.render(cache, ks.KnotSplats(p, knots, times), [3.0], [230e9], L, precision=ks.KS_MIXED))
+    assert rel(img[0, 0], ref) < 1e-4
+    cache.close()
+
+
 def test_fp64_pieces_of_rays():
     # 52900 rays x 2048 samples: two pieces of the FP64 stream and two of the adjoint's state
     p, N = wide_splats(4, 9), 2048
