@@ -29,18 +29,18 @@ sys.path.insert(0, ROOT)
 METRIC = "Stokes ray-samples/s (full-Stokes polarized transport)"
 UNIT = "ray-samples/s"
 
-# Algorithmic FP32-pipe work per event of the polarized consumer and the march (flops: add, mul =
+# Algorithmic FP32-pipe work per event of the polarized transport and the march (flops: add, mul =
 # 1, fma = 2, div = 1) and special-function-unit operations (sqrt, exp, log, sin, cos, atan, acos,
 # pow count 1 each), counted from the kernel source (kerrsplat_b200/csrc/ks_march.cuh,
-# ks_transfer.cuh, ks_lib.cu PolSink).
+# ks_transfer.cuh, ks_transport.cuh).
 FLOPS = {"samples": 330, "valid_samples": 95, "splat_tests": 22, "weights": 32, "coefficients": 170,
-         "frames": 115, "steps": 1150}
+         "frames": 115, "steps": 720}
 SFU = {"samples": 12, "valid_samples": 9, "splat_tests": 2, "weights": 1, "coefficients": 22, "frames": 4, "steps": 12}
 # k_transport's DRAM traffic per ray-sample: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch
-# of this workload at full size (256x256, N = 1024, 3 frequencies: 2.1709e9 + 0.1235e9 B over 65536 x 1024
+# on a scene of this workload's size (256x256, N = 1024, 3 frequencies: 1.5676e9 + 0.0602e9 B over 65536 x 1024
 # ray-samples; reads = the FP32 sample stream, 32 B per ray-sample, partly still in L2 after k_stream
 # writes it, + the plan; writes = segment states)
-CONSUME_TRAFFIC_PER_RAY_SAMPLE = (2.170923e9 + 0.123528e9) / (65536 * 1024)
+CONSUME_TRAFFIC_PER_RAY_SAMPLE = (1.567634e9 + 0.060244e9) / (65536 * 1024)
 
 
 def rank_info():

@@ -19,7 +19,7 @@
 // order and every unit has its own block of partial sums, so the gradient is the same bit for bit.
 //
 // Bound by instruction issue (41% of the issue slots at 12 warps per SM, its registers' limit). 224 x 224 x 896, 64 splats,
-// two frequencies: 10.6 ms; the step and element kernels before it took 28.7 ms. Four blocks per SM (128 registers) spill:
+// three frequencies: 11.1 ms; the step and element kernels before it took 28.7 ms. Four blocks per SM (128 registers) spill:
 // the whole gradient 23.6 ms against 22.5.
 #pragma once
 #include "ks_gradient.cuh"
