@@ -283,8 +283,8 @@ int ks_chi2_gradient_graph_launch(ks_context* ctx, int32_t wait);
 /* Release the captured graphs (the render's and the chi^2 + gradient evaluation's). */
 int ks_graph_destroy(ks_context* ctx);
 
-/* Test hook for the bounded waits (no reference counterpart): while on != 0, the mixed kernels arm
- * the shared-memory barrier of their splat-table staging without issuing the copy and poll it only
+/* Test hook for the bounded waits (no reference counterpart): while on != 0, the transport and
+ * reverse kernels of either precision arm the shared-memory barrier of their splat-table staging without issuing the copy and poll it only
  * 4096 times, and the tcgen05 GEMM arms its operand barriers without issuing the tile copies and gives
  * each wait ~10 ms, so every block's wait runs out; the kernels record it, free what they hold and
  * return (no fault, no hang) and the call fails with KS_ERR_TIMEOUT. The context stays usable; turn

@@ -926,8 +926,8 @@ int build_tables(ks_context* c, const ks_splat_set* sets, int nsets, int* ntot_o
     return KS_OK;
 }
 
-// A kernel's bounded wait that gave up (the device flag, cleared): KS_ERR_TIMEOUT. Bit 1: a mixed
-// kernel's table-staging copy; bit 2: a wait of the tcgen05 GEMM.
+// A kernel's bounded wait that gave up (the device flag, cleared): KS_ERR_TIMEOUT. Bit 1: the
+// table-staging copy of a transport or reverse kernel (either precision); bit 2: a wait of the tcgen05 GEMM.
 int check_device_flag(ks_context* c, const char* what) {
     unsigned f = 0;
     KS_CUDA(c, cudaMemcpy(&f, c->errflag.p, sizeof(unsigned), cudaMemcpyDeviceToHost));
@@ -1579,9 +1579,10 @@ struct VisData {
 
 namespace {
 
-__global__ void k_accumulate(double* __restrict__ dst, const double* __restrict__ src, long long n, int accumulate) {
+// dst is left as it was when a kernel before it gave up (`err`: the device flag)
+__global__ void k_accumulate(double* __restrict__ dst, const double* __restrict__ src, long long n, int accumulate, const unsigned* __restrict__ err) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q < n) dst[q] = (accumulate ? dst[q] : 0.0) + src[q];
+    if (q < n && *err == 0u) dst[q] = (accumulate ? dst[q] : 0.0) + src[q];
 }
 
 // Stage `count` elements of `src` (host or device) into `buf`; returns the device pointer.
@@ -1738,18 +1739,17 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
         }
     }
     cudaEventRecord(c->ev1, c->stream);
-    // 4. results
+    // 4. results; the gradient only if no kernel gave up
     const long long ng = (long long)ntot * GR_COUNT;
+    std::vector<double> hg;
     if (ng > 0) {
         if (is_device_ptr(dparams)) {
-            k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate);
+            k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate, c->errflag.as<unsigned>());
             c->launches++;
             KS_CUDA(c, cudaGetLastError());
         } else {
-            std::vector<double> hg(ng);
+            hg.resize(ng);
             KS_CUDA(c, cudaMemcpyAsync(hg.data(), c->dgrad.p, ng * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-            KS_CUDA(c, cudaStreamSynchronize(c->stream));
-            for (long long q = 0; q < ng; ++q) dparams[q] = (accumulate ? dparams[q] : 0.0) + hg[q];
         }
     }
     if (data && chi2_out) KS_CUDA(c, cudaMemcpyAsync(chi2_out, c->chi_val.p, sizeof(double), cudaMemcpyDefault, c->stream));
@@ -1762,7 +1762,9 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     c->adjoint_ms += ms;
-    if (precision != KS_FP64) return check_device_flag(c, "adjoint");
+    const int flag = check_device_flag(c, "adjoint");
+    if (flag) return flag;
+    for (size_t q = 0; q < hg.size(); ++q) dparams[q] = (accumulate ? dparams[q] : 0.0) + hg[q];
     return KS_OK;
 }
 
@@ -1839,7 +1841,7 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
         status = launch_reverse(c, ntot, nmax, false, false);
     const long long ng = (long long)ntot * GR_COUNT;
     if (status == KS_OK && ng > 0) {
-        k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate);
+        k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate, c->errflag.as<unsigned>());
         if (cudaGetLastError() != cudaSuccess) status = fail(c, KS_ERR_DEVICE, "graph capture: gradient");
     }
     if (status == KS_OK && cudaMemcpyAsync(chi2, c->chi_val.p, sizeof(double), cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
