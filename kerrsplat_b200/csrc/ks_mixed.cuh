@@ -14,20 +14,20 @@ constexpr double kQCUT = 13.815510557964274;   // -ln(WEIGHT_CUTOFF): G > 1e-6 <
 constexpr int kMaxSplatWords = 16;              // the FP32 transport takes up to 512 splats
 
 // The bounds of a work unit's samples (quasi-Cartesian KS box, cylindrical radius and height, and the
-// range of their emission times t = t_obs - t~) and the splats whose support can reach them: a
+// range of their lookback times) and the splats whose support can reach them: a
 // pattern-rotating splat's support lies within its support radius of the circle its centre runs on
 // (rho = ST_RHO, z = ST_CZ), and within it of the arc its centre covers over the unit's emission times
 // (the centre's angle is phi_0 + omega (t - t0)); a knot splat's within its bounding sphere (centre
 // ST_CX..CZ, radius^2 ST_RHO). Splats outside are below the weight cutoff at every sample of the unit,
 // so the per-sample tests skip them (the same result, fewer tests).
-struct UnitBox { float xlo, xhi, ylo, yhi, zlo, zhi, rlo, rhi, tlo, thi; };
+struct UnitBox { float xlo, xhi, ylo, yhi, zlo, zhi, rlo, rhi, slo, shi; };
 
-// Widen the unit box with one sample (position, cylindrical radius, emission time).
-__device__ __forceinline__ void unit_box_add(UnitBox& b, float x, float y, float z, float t) {
+// Widen the unit box with one sample (position, cylindrical radius, lookback time).
+__device__ __forceinline__ void unit_box_add(UnitBox& b, float x, float y, float z, float s) {
     const float rho = sqrtf(x * x + y * y);
     b.xlo = fminf(b.xlo, x); b.xhi = fmaxf(b.xhi, x); b.ylo = fminf(b.ylo, y); b.yhi = fmaxf(b.yhi, y);
     b.zlo = fminf(b.zlo, z); b.zhi = fmaxf(b.zhi, z); b.rlo = fminf(b.rlo, rho); b.rhi = fmaxf(b.rhi, rho);
-    b.tlo = fminf(b.tlo, t); b.thi = fmaxf(b.thi, t);
+    b.slo = fminf(b.slo, s); b.shi = fmaxf(b.shi, s);
 }
 __device__ __forceinline__ UnitBox unit_box_empty() { return {3e38f, -3e38f, 3e38f, -3e38f, 3e38f, -3e38f, 3e38f, -3e38f, 3e38f, -3e38f}; }
 
@@ -69,7 +69,7 @@ __device__ __forceinline__ float table_reach2(const TAB* tab, int ntot, float* s
 __device__ __forceinline__ void unit_box_reduce(UnitBox& b) {
     b.xlo = warp_min(b.xlo); b.xhi = warp_max(b.xhi); b.ylo = warp_min(b.ylo); b.yhi = warp_max(b.yhi);
     b.zlo = warp_min(b.zlo); b.zhi = warp_max(b.zhi); b.rlo = warp_min(b.rlo); b.rhi = warp_max(b.rhi);
-    b.tlo = warp_min(b.tlo); b.thi = warp_max(b.thi);
+    b.slo = warp_min(b.slo); b.shi = warp_max(b.shi);
 }
 
 // ---- TMA bulk staging ----------------------------------------------------------------------------

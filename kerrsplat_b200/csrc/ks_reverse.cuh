@@ -418,7 +418,7 @@ k_reverse(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ rows
                     if (lane == 0) ball[kl] = bl;
                     if (act) {
                         const T* p = sp + (long long)kl * SM_COUNT * fs;
-                        unit_box_add(b, float(p[SM_X * fs]), float(p[SM_Y * fs]), float(p[SM_Z * fs]), float(t_obs - p[SM_T * fs]));
+                        unit_box_add(b, float(p[SM_X * fs]), float(p[SM_Y * fs]), float(p[SM_Z * fs]), float(p[SM_T * fs]));
                     }
                 }
                 unit_box_reduce(b);
@@ -435,11 +435,11 @@ k_reverse(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ rows
                     const float* o = boxes + q * 10;
                     b.xlo = fminf(b.xlo, o[0]); b.xhi = fmaxf(b.xhi, o[1]); b.ylo = fminf(b.ylo, o[2]); b.yhi = fmaxf(b.yhi, o[3]);
                     b.zlo = fminf(b.zlo, o[4]); b.zhi = fmaxf(b.zhi, o[5]); b.rlo = fminf(b.rlo, o[6]); b.rhi = fmaxf(b.rhi, o[7]);
-                    b.tlo = fminf(b.tlo, o[8]); b.thi = fmaxf(b.thi, o[9]);
+                    b.slo = fminf(b.slo, o[8]); b.shi = fmaxf(b.shi, o[9]);
                 }
                 for (int wd = warp - g0; wd < nw; wd += G) {
                     const int i = wd * 32 + lane;
-                    const unsigned m = __ballot_sync(0xffffffffu, i < ntot && b.xlo <= b.xhi && row_reaches(rows + (long long)i * ST, b));
+                    const unsigned m = __ballot_sync(0xffffffffu, i < ntot && b.xlo <= b.xhi && row_reaches(rows + (long long)i * ST, b, t_obs));
                     if (lane == 0) cand[g0 / G * nw + wd] = m;
                 }
             }

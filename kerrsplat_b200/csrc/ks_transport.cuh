@@ -589,28 +589,32 @@ __device__ __forceinline__ void get16(const double* p, double* v) {
 
 // ---- candidates ------------------------------------------------------------------------------------------
 
-// Whether row r's support can reach the box (unit_candidates' bounds: the circle or the arc the centre runs
-// on, or a knot splat's bounding sphere).
+// Whether row r's support can reach the box at the observation time: the circle, then the arc, that the centre runs
+// on, or a knot splat's bounding sphere. The box and this test are FP32 in either precision. The box holds lookback
+// times and the phase is formed from t_obs - t0, taken in T, so that what is rounded are differences of times: in FP32
+// a time of 1e7 is off by 0.5. Positions are padded by a few of their roundings.
 template <class T>
-__device__ __forceinline__ bool row_reaches(const T* r, const UnitBox& b) {
+__device__ __forceinline__ bool row_reaches(const T* r, const UnitBox& b, T t_obs) {
     const float cz = float(r[RW_CZ]), rho = float(r[RW_RHO]);
     if (int(r[RW_KIND]) == KS_KNOT21) {
-        const float cx = float(r[RW_CX]), cy = float(r[RW_CY]);
-        const float dx = fmaxf(fmaxf(b.xlo - cx, cx - b.xhi), 0.f);
-        const float dy = fmaxf(fmaxf(b.ylo - cy, cy - b.yhi), 0.f);
-        const float dz = fmaxf(fmaxf(b.zlo - cz, cz - b.zhi), 0.f);
+        const float cx = float(r[RW_CX]), cy = float(r[RW_CY]), e = 1e-6f * (fabsf(cx) + fabsf(cy) + fabsf(cz));
+        const float dx = fmaxf(fmaxf(b.xlo - cx, cx - b.xhi) - e, 0.f);
+        const float dy = fmaxf(fmaxf(b.ylo - cy, cy - b.yhi) - e, 0.f);
+        const float dz = fmaxf(fmaxf(b.zlo - cz, cz - b.zhi) - e, 0.f);
         return dx * dx + dy * dy + dz * dz <= rho * 1.0001f;
     }
-    const float supp = float(r[RW_SUPP]) * 1.0001f;
-    const float dr = fmaxf(fmaxf(b.rlo - rho, rho - b.rhi), 0.f);
-    const float dz = fmaxf(fmaxf(b.zlo - cz, cz - b.zhi), 0.f);
+    const float supp = float(r[RW_SUPP]) * 1.0001f, e = 1e-6f * (rho + fabsf(cz));
+    const float dr = fmaxf(fmaxf(b.rlo - rho, rho - b.rhi) - e, 0.f);
+    const float dz = fmaxf(fmaxf(b.zlo - cz, cz - b.zhi) - e, 0.f);
     if (!(dr * dr + dz * dz <= supp)) return false;
-    const float om = float(r[RW_OMEGA]), t0 = float(r[RW_T0]);
-    const float pa = om * (b.tlo - t0), pb = om * (b.thi - t0);
-    // the pad covers the FP32 rounding of the angles (phases up to ~1e3 rad) and positions
-    const float pad = 1e-3f * rho + 1e-4f * (fabsf(pa) + fabsf(pb)) * rho + 1e-3f;
+    const float om = float(r[RW_OMEGA]), off = float(t_obs - r[RW_T0]);
+    const float pa = om * (off - b.shi), pb = om * (off - b.slo);
+    // the pad covers the FP32 rounding of the angles (phases up to ~1e3 rad) and positions, and in FP32 that of the
+    // times a sample is tested at
+    float pad = 1e-3f * rho + 1e-4f * (fabsf(pa) + fabsf(pb)) * rho + 1e-3f;
+    if (sizeof(T) == 4) pad += 2.4e-7f * fabsf(om) * rho * (fabsf(float(t_obs)) + fabsf(float(r[RW_T0])));
     const float lo = fminf(pa, pb), hi = fmaxf(pa, pb);
-    if (!(b.tlo <= b.thi) || !(hi - lo < 6.0f)) return true;
+    if (!(b.slo <= b.shi) || !(hi - lo < 6.0f)) return true;
     const float A = float(r[RW_ANG]) + lo, B = float(r[RW_ANG]) + hi;
     float sa, ca, sb, cb;
     sincosf(A, &sa, &ca);
@@ -761,7 +765,7 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                     if (!(stream_flags(p[SM_FLAGS * fs]) & 8u)) continue;
                     const T x = p[SM_X * fs], yy = p[SM_Y * fs], z = p[SM_Z * fs];
                     if (x * x + yy * yy + z * z > reach2) continue;   // beyond every splat: no candidate needed
-                    unit_box_add(b, float(x), float(yy), float(z), float(t_obs - p[SM_T * fs]));
+                    unit_box_add(b, float(x), float(yy), float(z), float(p[SM_T * fs]));
                 }
                 unit_box_reduce(b);
                 const float* bf = reinterpret_cast<const float*>(&b);
@@ -777,11 +781,11 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                     const float* o = boxes + q * 10;
                     b.xlo = fminf(b.xlo, o[0]); b.xhi = fmaxf(b.xhi, o[1]); b.ylo = fminf(b.ylo, o[2]); b.yhi = fmaxf(b.yhi, o[3]);
                     b.zlo = fminf(b.zlo, o[4]); b.zhi = fmaxf(b.zhi, o[5]); b.rlo = fminf(b.rlo, o[6]); b.rhi = fmaxf(b.rhi, o[7]);
-                    b.tlo = fminf(b.tlo, o[8]); b.thi = fmaxf(b.thi, o[9]);
+                    b.slo = fminf(b.slo, o[8]); b.shi = fmaxf(b.shi, o[9]);
                 }
                 for (int wd = warp - g0; wd < nw; wd += G) {
                     const int i = wd * 32 + lane;
-                    const bool keep = i < ntot && b.xlo <= b.xhi && row_reaches(rows + (long long)i * ST, b);
+                    const bool keep = i < ntot && b.xlo <= b.xhi && row_reaches(rows + (long long)i * ST, b, t_obs);
                     const unsigned m = __ballot_sync(0xffffffffu, keep);
                     if (lane == 0) cand[g0 / G * nw + wd] = m;
                 }

@@ -57,3 +57,49 @@ def test_a_staging_wait_that_runs_out_is_reported(call, precision):
     if call != "render":
         assert not (np.all(held == 3.0) and bool((dev == 3.0).all()))
     cache.close()
+
+
+@pytest.mark.parametrize("shift", [1e6, 1e8])
+def test_fp64_times_far_from_zero(shift):
+    """The same scene at times `shift` later: an FP64 time there is rounded by 1e-16 of it, some 1e-8 M, which moves a
+    centre by 1e-8 M and a weight by 1e-7 at most; 1e-6 is allowed."""
+    rng = np.random.Generator(np.random.PCG64(21))
+    p = scenes.thermal_params(rng, 40, A, rlo=3.0, rhi=8.0)
+    p[3:6] = np.log(rng.uniform(0.2, 0.4, (3, 40)))
+    p[10], p[11] = rng.uniform(-20.0, 20.0, 40), np.log(1e9)
+    later = p.copy(order="F")
+    later[10] += shift
+    cache = cache_of(24, 22, 128)
+    img = np.asarray(ks.render(cache, ks.PolarizedSplats(p), [4.0], [230e9], L))
+    assert np.abs(img).max() > 0
+    assert rel(ks.render(cache, ks.PolarizedSplats(later), [4.0 + shift], [230e9], L), img) < 1e-6
+    ds = rng.standard_normal(img.shape)
+    g = ks.adjoint(cache, ks.PolarizedSplats(p), [4.0], [230e9], L, ds)
+    h = ks.adjoint(cache, ks.PolarizedSplats(later), [4.0 + shift], [230e9], L, ds)
+    for row in range(21):
+        assert np.linalg.norm(h[row] - g[row]) <= 1e-6 * max(np.linalg.norm(g[row]), 1e-6 * np.linalg.norm(g)), row
+    cache.close()
+
+
+def test_fp64_samples_at_the_edge_of_a_support(oracle):
+    """A narrow splat above the outermost sample of one ray, that sample a little inside the weight cutoff (1e-6), where
+    the FP32 rounding of a height of some 1000 M (1e-4 M) is more than the distance to the edge: it shows in FP64 on
+    every ray. An oracle sample lies up to 1e-9 M from the library's, 5e-7 of a weight: 1e-5 is allowed."""
+    q = np.sqrt(1.0 - A * A)
+    for beta in np.linspace(3.1, 9.7, 12):
+        cam = ks.Camera(np.array([1.3]), np.array([beta]))
+        cache = ks.regenerate(ks.GeodesicCache(cam, 256), A, THO)
+        s = cache.samples()
+        assert s["flags"][0, 0] & 1
+        r, th, ph = s["r"][0, 0], s["theta"][0, 0], s["phi"][0, 0]
+        ph = ph + A / (2 * q) * np.log((r - 1 - q) / (r - 1 + q)) - np.arctan2(A, r)   # the azimuth of the splats' frame
+        p = wide_splats(1, 23)
+        p[3:6] = np.log(0.01)
+        p[20], p[11], p[12] = 0.0, np.log(1e9), np.log(1e12)
+        p[0:3, 0] = r * np.array([np.sin(th) * np.cos(ph), np.sin(th) * np.sin(ph), np.cos(th)])
+        p[2] += 0.01 * np.sqrt(2 * 13.8149)   # the weight's exponent at the sample; the cutoff's is 13.8155
+        img = np.asarray(ks.render(cache, ks.PolarizedSplats(p), [0.0], [230e9], L))[0, 0]
+        ref = oracle.polarized_image(A, THO, cam.alpha, cam.beta, 256, 64, [("thermal", p, None)], 0.0, 230e9, L)
+        assert np.linalg.norm(ref) > 0
+        assert rel(img, ref) < 1e-5, beta
+        cache.close()
