@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/kerrsplat_b200.h"
@@ -30,6 +31,7 @@ struct DevBuf {
         return e;
     }
     void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+    void swap(DevBuf& o) { std::swap(p, o.p); std::swap(n, o.n); }
     template <class U> U* as() const { return reinterpret_cast<U*>(p); }
 };
 
@@ -58,6 +60,8 @@ struct ks_context {
     cudaGraph_t cgraph = nullptr;         // ks_chi2_gradient_graph_capture: one mixed chi^2 + gradient evaluation
     cudaGraphExec_t cgraph_exec = nullptr;
     std::vector<void*> cgraph_bufs;
+    // what a captured graph reads of its own call: the splat table with the knots, the times and the frequencies
+    DevBuf graph_tab, graph_combos, cgraph_tab, cgraph_combos;
     bool capturing = false;               // inside that capture: no timing events
     int stage_test = 0;                   // ks_set_stage_test
     std::vector<void*> graph_bufs;        // the buffers the graph uses, as captured (a replay checks them)

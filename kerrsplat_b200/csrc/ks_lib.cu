@@ -1433,8 +1433,8 @@ int ks_riaf_image(ks_context* c, const double* model, int32_t pandya, const doub
 
 // The device buffers a captured render reads or writes (a replay requires them unmoved).
 std::vector<void*> graph_buffers(const ks_context* c) {
-    return {c->tab.p, c->tab32.p, c->rows.p, c->kstop.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->combos.p, c->errflag.p,
-            c->perm.p, c->plan.p, c->anchors.p, c->aoff.p};
+    return {c->tab32.p, c->rows.p, c->kstop.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->errflag.p, c->perm.p,
+            c->plan.p, c->anchors.p, c->aoff.p};
 }
 
 void release_graph(cudaGraph_t& g, cudaGraphExec_t& ex) {
@@ -1451,6 +1451,23 @@ std::vector<void*> chi2_graph_buffers(const ks_context* c) {
                             &c->chi_val, &c->dgrad})
         b.push_back(d->p);
     return b;
+}
+
+// A capture's own copies of its call's splat table (whose knots stay as they are) and of its times and frequencies: every
+// later call writes its own into the context's buffers. In the context's place while it exists.
+struct GraphInputs {
+    ks_context* c;
+    DevBuf &tab, &combos;
+    GraphInputs(ks_context* c_, DevBuf& t, DevBuf& s) : c(c_), tab(t), combos(s) { c->tab.swap(tab); c->combos.swap(combos); }
+    ~GraphInputs() { c->tab.swap(tab); c->combos.swap(combos); }
+};
+int copy_graph_inputs(ks_context* c, DevBuf& tab, DevBuf& combos, int ntot, int nframes, int nfreq) {
+    const size_t nt = (size_t(std::max(ntot, 1)) * ST_COUNT + c->nkv) * sizeof(double), nc = (size_t(nframes) + nfreq) * sizeof(double);
+    KS_CUDA(c, tab.ensure(nt));
+    KS_CUDA(c, combos.ensure(nc));
+    KS_CUDA(c, cudaMemcpyAsync(tab.p, c->tab.p, nt, cudaMemcpyDeviceToDevice, c->stream));
+    KS_CUDA(c, cudaMemcpyAsync(combos.p, c->combos.p, nc, cudaMemcpyDeviceToDevice, c->stream));
+    return KS_OK;
 }
 
 // The splat tables of device-resident sets rebuilt on the device inside a capture (the knot array
@@ -1507,6 +1524,8 @@ int ks_render_graph_capture(ks_context* c, const ks_splat_set* sets, int32_t nse
         ntot += sets[s].nsplat;
         thermal_only = thermal_only && (sets[s].kind == KS_THERMAL21 || sets[s].nsplat == 0);
     }
+    if ((status = copy_graph_inputs(c, c->graph_tab, c->graph_combos, ntot, nframes, nfreq))) return status;
+    GraphInputs own(c, c->graph_tab, c->graph_combos);
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
     status = capture_tables(c, sets, nsets, ntot, false);
@@ -1551,6 +1570,7 @@ int ks_graph_destroy(ks_context* c) {
     if (!c) return KS_ERR_ARGUMENT;
     release_graph(c->graph, c->graph_exec);
     release_graph(c->cgraph, c->cgraph_exec);
+    for (DevBuf* d : {&c->graph_tab, &c->graph_combos, &c->cgraph_tab, &c->cgraph_combos}) d->release();
     return KS_OK;
 }
 
@@ -1818,6 +1838,8 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
     const long long nrc = n * ncombo;
     const long long nblk = (nrc + 255) / 256;
     const size_t rows = size_t(ncombo) * c->st.N * c->npad;
+    if ((status = copy_graph_inputs(c, c->cgraph_tab, c->cgraph_combos, ntot, nframes, nfreq))) return status;
+    GraphInputs own(c, c->cgraph_tab, c->cgraph_combos);
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
     status = capture_tables(c, sets, nsets, ntot, true);

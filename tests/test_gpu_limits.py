@@ -103,3 +103,32 @@ def test_fp64_samples_at_the_edge_of_a_support(oracle):
         assert np.linalg.norm(ref) > 0
         assert rel(img, ref) < 1e-5, beta
         cache.close()
+
+
+def test_graph_replays_keep_their_own_call():
+    """A captured graph renders the frames, frequencies and knots of its capture whatever calls came between, of the
+    same sizes (nothing is reallocated) and of other layouts (J v)."""
+    import torch
+    cache, cuda = cache_of(16, 14, 96), lambda p: torch.tensor(p, device="cuda")
+    p, kt = wide_splats(6, 24), np.linspace(-40.0, 60.0, 5)
+    knots = scenes.trajectory_knots(p, A, kt)
+    other = np.asarray(knots) * 1.2
+    thermal = ks.PolarizedSplats(cuda(p))
+    data = cuda(np.random.Generator(np.random.PCG64(25)).standard_normal((2, 1, cache.npix, 4)) * 1e-6)
+    def between(knots, t, nus):
+        img = ks.render(cache, ks.KnotSplats(cuda(p), knots, kt), [t], nus, L, precision=ks.KS_MIXED).cpu().numpy()
+        ks.jvp(cache, thermal, [t], nus, L, np.ones((1, 21, 6)), precision=ks.KS_MIXED)
+        ks.chi2_gradient(cache, thermal, [t], nus, L, data, 1e-7, precision=ks.KS_MIXED)
+        return img
+
+    between(knots, 0.0, [230e9, 86e9])   # the buffers have their sizes
+    gc = ks.capture_chi2_gradient(cache, thermal, [0.0], [230e9, 86e9], L, data, 1e-7)
+    g = ks.capture_render(cache, ks.KnotSplats(cuda(p), knots, kt), [0.0], [230e9, 86e9], L)
+    first = g.replay().cpu().numpy().copy()
+    chi2, grad = [x.cpu().numpy().copy() for x in gc.replay()]
+    assert np.abs(first).max() > 0 and np.abs(grad).max() > 0
+    assert not np.array_equal(between(other, 50.0, [345e9, 43e9]), first)
+    assert np.array_equal(g.replay().cpu().numpy(), first)
+    again = [x.cpu().numpy() for x in gc.replay()]
+    assert np.array_equal(again[0], chi2) and np.array_equal(again[1], grad)
+    cache.close()
