@@ -163,9 +163,10 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     }
     constexpr int B128 = 4, B256 = 2;
     Shape s128 = transport_shape<float, CH, KM, 128>(ntot, c->nkv, c->st.N, B128), s256 = transport_shape<float, CH, KM, 256>(ntot, c->nkv, c->st.N, B256);
-    // the largest table (splat constants and knots) a call may bring, by the frequencies of a unit; its rows stay in global
-    // memory where a block's shared memory does not hold them
-    if (((size_t)ntot * ST_COUNT + c->nkv) * sizeof(float) > 227 * 1024 - 4 * (5848 + 4096 * size_t(CH))) s128.blocks = s256.blocks = 0;
+    // the largest table (splat constants and knots) a call may bring, by its frequencies (four or more as many as two); its
+    // rows stay in global memory where a block's shared memory does not hold them
+    constexpr int kBound = CH == 4 ? 2 : CH;
+    if (((size_t)ntot * ST_COUNT + c->nkv) * sizeof(float) > 227 * 1024 - 4 * (5848 + 4096 * size_t(kBound))) s128.blocks = s256.blocks = 0;
     if (s128.blocks == 0 && s256.blocks == 0) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
     // the wider block where shared memory (a large table) holds more of its warps, or the autotuner's choice
     bool wide = s256.blocks * 8 > s128.blocks * 4;

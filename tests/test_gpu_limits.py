@@ -132,3 +132,28 @@ def test_graph_replays_keep_their_own_call():
     again = [x.cpu().numpy() for x in gc.replay()]
     assert np.array_equal(again[0], chi2) and np.array_equal(again[1], grad)
     cache.close()
+
+
+@pytest.mark.parametrize("nf,values", [(1, 48168), (2, 44072), (3, 39976), (4, 44072), (5, 44072)])
+def test_largest_tables_by_frequencies(nf, values):
+    """The largest FP32 table (51 values a splat and four a knot) at each number of frequencies is taken, one knot more
+    is refused. Four frequencies take what two do. The image is that of the frequencies by themselves: 1e-4 is the FP32
+    transport's budget."""
+    n = 256
+    nk = (values // n - 51) // 4
+    p = wide_splats(n, 26)
+    p[3:6] -= 1.0
+    cache, nus = cache_of(7, 6, 40), np.geomspace(86e9, 690e9, 5)[:nf]
+
+    def model(nk):
+        t = np.linspace(-60.0, 40.0, nk)
+        return ks.KnotSplats(p, scenes.trajectory_knots(p, A, t), t)
+
+    with pytest.raises(ValueError, match="too many splats"):
+        ks.render(cache, model(nk + 1), [3.0], nus, L, precision=ks.KS_MIXED)
+    m = model(nk)
+    img = np.asarray(ks.render(cache, m, [3.0], nus, L, precision=ks.KS_MIXED))
+    assert np.abs(img).max() > 0
+    for v in range(nf):
+        assert rel(img[v], np.asarray(ks.render(cache, m, [3.0], nus[v:v + 1], L, precision=ks.KS_MIXED))[0]) < 1e-4
+    cache.close()
