@@ -25,6 +25,13 @@ def wide_splats(n, seed):
     return p
 
 
+def orbit_knots(p, times):
+    """The centres of `p` on their pattern circles at `times`, (3, times, splats)."""
+    ang = np.arctan2(p[1], p[0]) + p[20] * np.asarray(times)[:, None]
+    rho = np.hypot(p[0], p[1])
+    return np.stack([rho * np.cos(ang), rho * np.sin(ang), np.broadcast_to(p[2], ang.shape)])
+
+
 def cache_of(na, nb, N):
     return ks.regenerate(ks.GeodesicCache(ks.Camera((-8.9, 9.3), (-9.1, 8.7), (na, nb)), N), A, THO)
 
@@ -111,7 +118,7 @@ def test_graph_replays_keep_their_own_call():
     import torch
     cache, cuda = cache_of(16, 14, 96), lambda p: torch.tensor(p, device="cuda")
     p, kt = wide_splats(6, 24), np.linspace(-40.0, 60.0, 5)
-    knots = scenes.trajectory_knots(p, A, kt)
+    knots = orbit_knots(p, kt)
     other = np.asarray(knots) * 1.2
     thermal = ks.PolarizedSplats(cuda(p))
     data = cuda(np.random.Generator(np.random.PCG64(25)).standard_normal((2, 1, cache.npix, 4)) * 1e-6)
@@ -147,7 +154,7 @@ def test_largest_tables_by_frequencies(nf, values):
 
     def model(nk):
         t = np.linspace(-60.0, 40.0, nk)
-        return ks.KnotSplats(p, scenes.trajectory_knots(p, A, t), t)
+        return ks.KnotSplats(p, orbit_knots(p, t), t)
 
     with pytest.raises(ValueError, match="too many splats"):
         ks.render(cache, model(nk + 1), [3.0], nus, L, precision=ks.KS_MIXED)
