@@ -106,7 +106,7 @@ __device__ __forceinline__ void thermal_row_bar(const T* r, T ne, T nu, T st, T 
     const T s20 = hrcp(T(1) + q20), sw = lo ? q20 * s20 : s20, sw1 = lo ? s20 : q20 * s20;   // sw1 = 1 - sw
     const T lx = hlog2(x + T(1e-16));
     const T ex = T(0.011) * hexp(x * T(-1.0 / 47.2)), exl = ex * x * T(1.0 / 47.2);
-    const T px = T(7.9370052598409974e-01 / 67.44733739010397 * 3.141592653589793 * 1e4) * hexp2(T(-8.0 / 3) * lx);
+    const T px = T(7.9370052598409974e-01 / 67.44733739010397 * 3.141592653589793 * 1e4) * hexp2(fmin(T(-8.0 / 3) * lx, T(100)));
     const T x1 = hexp2(T(1.035) * lx) * T(1.0 / 4.7), e1 = T(2.011) * hexp(-x1);
     const T x2 = hexp2(T(1.2) * lx) * T(1.0 / 2.73), e2 = hexp(-x2);
     T sh, ch;
@@ -140,9 +140,8 @@ __device__ __forceinline__ void thermal_row_bar(const T* r, T ne, T nu, T st, T 
     constexpr double kY = kHPL / (kME * kCL * kCL), kB = 2.0 * kHPL / (kCL * kCL);
     const T y = T(kY) * nu * iT;
     const T em1 = y < T(2e-3) ? y * (T(1) + y * (T(0.5) + y * (T(1.0 / 6) + y * T(1.0 / 24)))) : expm1(y);
-    const T nh0 = nu * T(1e-11), bn = T(kB * 1e33) * nh0 * nh0 * nh0;
-    const T iB = bn > T(0) ? em1 * hrcp(bn) : T(0);
-    const T ry = y * (em1 + T(1)) * hrcp(em1);                   // d ln(1 / B) / d ln y
+    const T iB = planck_inverse(T(kB * 1e33), nu, em1);
+    const T ry = y + y * hrcp(em1);                              // d ln(1 / B) / d ln y
     // the cap (coefficients.jl:264-288): jQ, jV scaled by 0.99 jI / sqrt(jQ^2 + jV^2) where that is below one
     T cap = T(1), qq = T(0), vv = T(0), ip2 = T(0);              // ip2 != 0: capped; jQ / jI, jV / jI, 1 / (their squares' sum)
     if (jI >= smallest<T>()) {

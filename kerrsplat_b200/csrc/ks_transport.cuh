@@ -289,6 +289,14 @@ __device__ __forceinline__ T row_cap(T I, T Q, T V) {
     return p2 > T(0.9801) ? T(0.99) * hrsqrt(p2) : T(1);
 }
 
+// 1 / B_nu from exp(h nu / k T) - 1; zero where that, or its product with what follows, would overflow: a splat far too
+// cold to emit, whose absorptivity is 0 / 0
+template <class T>
+__device__ __forceinline__ T planck_inverse(T k, T nu, T em1) {
+    const T nh = nu * T(1e-11), bn = k * nh * nh * nh, i = em1 * hrcp(bn);
+    return bn > T(0) && i < (sizeof(T) == 4 ? T(1e30) : T(1e300)) ? i : T(0);
+}
+
 // The thermal fits (thermal_cs, coefficients.jl:101-145): the powers of x and of nu / nu_s from one logarithm
 // each, the constants folded in FP64, and one cap for the emissivities and the absorptivities (Kirchhoff's law
 // gives both the same ratios). Returns false where nothing emits, absorbs or rotates.
@@ -310,7 +318,7 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     const T s20 = hrcp(T(1) + q20), sw = lo ? q20 * s20 : s20;   // 0.5 + 0.5 tanh((ln x - ln 120) / 0.1)
     const T lx = hlog2(x + T(1e-16));
     const T ex = hexp(x * T(-1.0 / 47.2));
-    const T extra = (T(0.011) * ex - T(7.9370052598409974e-01 / 67.44733739010397 * 3.141592653589793 * 1e4) * hexp2(T(-8.0 / 3) * lx)) * sw;
+    const T extra = (T(0.011) * ex - T(7.9370052598409974e-01 / 67.44733739010397 * 3.141592653589793 * 1e4) * hexp2(fmin(T(-8.0 / 3) * lx, T(100)))) * sw;   // the bound: sw is zero long before
     const T jf = T(2.011) * hexp(hexp2(T(1.035) * lx) * T(-1.0 / 4.7)) - fcos(x * T(0.5)) * hexp(hexp2(T(1.2) * lx) * T(-1.0 / 2.73)) - T(0.011) * ex + extra;
     const T plb = pl * b;
     c[6] = T(0.5 * kRV) * nu * (jf * plb * b * (r[RW_KR] + T(6) * Te) * st * st);
@@ -331,8 +339,7 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     if (y < T(2e-3)) em1 = y * (T(1) + y * (T(0.5) + y * (T(1.0 / 6) + y * T(1.0 / 24))));
     else if constexpr (sizeof(T) == 4) em1 = expm1f(y);
     else em1 = expm1(y);
-    const T nh0 = nu * T(1e-11), bn = T(kB * 1e33) * nh0 * nh0 * nh0;
-    const T iB = bn > T(0) ? em1 * hrcp(bn) : T(0);
+    const T iB = planck_inverse(T(kB * 1e33), nu, em1);
     const T cap = row_cap(jI, jQ, jV);
     c[0] = jI; c[1] = jQ * cap; c[2] = jV * cap;
     c[3] = jI * iB; c[4] = c[1] * iB; c[5] = c[2] * iB;

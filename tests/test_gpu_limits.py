@@ -164,3 +164,25 @@ def test_largest_tables_by_frequencies(nf, values):
     for v in range(nf):
         assert rel(img[v], np.asarray(ks.render(cache, m, [3.0], nus[v:v + 1], L, precision=ks.KS_MIXED))[0]) < 1e-4
     cache.close()
+
+
+@pytest.mark.parametrize("ln_te", [-21.0, -22.0, -24.0, -25.5, -28.0, -32.0])
+def test_splats_too_cold_to_emit(oracle, ln_te):
+    """Beside ordinary splats, cold ones, where exp(h nu / k T) overflows in FP32 or FP64, only rotate the polarization,
+    in the limit T = 0 the same whatever T is: 6 T, 5e-9 of a rotativity at the warmest, so FP64 agrees with the
+    oracle's image at the warmest (the others are 0 / 0 to it) to 1e-8; FP32 with FP64 as elsewhere, 1e-4 and 1e-3."""
+    p = wide_splats(6, 27)
+    p[13, ::2] = ln_te
+    warm = p.copy(order="F")
+    warm[13, ::2] = -21.0
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), (9, 7))
+    cache, m = cache_of(9, 7, 70), ks.PolarizedSplats(p)
+    img = np.asarray(ks.render(cache, m, [0.0], [230e9], L))
+    ref = oracle.polarized_image(A, THO, cam.alpha, cam.beta, 70, 64, [("thermal", warm, None)], 0.0, 230e9, L)
+    assert rel(img[0, 0], ref) < 1e-8
+    ds = np.random.Generator(np.random.PCG64(28)).standard_normal(img.shape)
+    g = ks.adjoint(cache, m, [0.0], [230e9], L, ds)
+    assert np.all(np.isfinite(g))
+    assert rel(ks.render(cache, m, [0.0], [230e9], L, precision=ks.KS_MIXED), img) < 1e-4
+    assert rel(ks.adjoint(cache, m, [0.0], [230e9], L, ds, precision=ks.KS_MIXED), g) < 1e-3
+    cache.close()
