@@ -129,8 +129,8 @@ __device__ __forceinline__ void thermal_row_bar(const T* r, T ne, T nu, T st, T 
     const T ls = hlog2(nu * hrcp(nus)) * T(1.0 / 3);
     const T c13 = hexp2(-ls), c23 = c13 * c13, u = T(1.8899 / 3) * hexp2(ls);
     const T e13 = hexp(T(-3) * u);
-    constexpr double kJ = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);
-    const T iT = hrcp(Te), ist = hrcp(st), pj = T(kJ) * ne * nu * iT * iT * e13, pI = pj * T(2.5651);
+    constexpr double kJ = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);   // times nu first: 2e-30 n_e underflows in FP32
+    const T iT = hrcp(Te), ist = hrcp(st), pj = T(kJ) * nu * ne * iT * iT * e13, pI = pj * T(2.5651);
     const T fI = T(1) + T(1.92) * c13 + T(0.9977) * c23, fIx = T(-1.92 / 3) * c13 - T(0.9977 * 2 / 3) * c23;
     const T fQ = T(1) + T(0.93193) * c13 + T(0.499873) * c23, fQx = T(-0.93193 / 3) * c13 - T(0.499873 * 2 / 3) * c23;
     const T v1 = T(1.81384) * nus * inu, v2 = T(3.42319) * c23, v3 = T(0.0292545) * hexp2(T(-1.5) * ls), v4 = T(2.03773) * c13;
@@ -144,9 +144,11 @@ __device__ __forceinline__ void thermal_row_bar(const T* r, T ne, T nu, T st, T 
     const T ry = y + y * hrcp(em1);                              // d ln(1 / B) / d ln y
     // the cap (coefficients.jl:264-288): jQ, jV scaled by 0.99 jI / sqrt(jQ^2 + jV^2) where that is below one
     T cap = T(1), qq = T(0), vv = T(0), ip2 = T(0);              // ip2 != 0: capped; jQ / jI, jV / jI, 1 / (their squares' sum)
-    if (jI >= smallest<T>()) {
-        const T iI = hrcp(jI);
-        qq = jQ * iI; vv = jV * iI;
+    if (jI > T(0)) {
+        T I = jI, Q = jQ, V = jV;
+        scale_small(I, Q, V);
+        const T iI = hrcp(I);
+        qq = Q * iI; vv = V * iI;
         const T p2 = qq * qq + vv * vv;
         if (p2 > T(0.9801)) {
             cap = T(0.99) * hrsqrt(p2);

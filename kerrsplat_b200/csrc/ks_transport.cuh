@@ -281,10 +281,19 @@ __device__ __forceinline__ LFrame<T> row_frame(const SampleFrame<T>& F, const T*
 // The smallest normal number: below it the hardware reciprocal is infinite.
 template <class T> __device__ __forceinline__ constexpr T smallest() { return sizeof(T) == 4 ? T(1.17549435e-38) : T(2.2250738585072014e-308); }
 
-// cap_factor (coefficients.jl:264-288) from the ratios to the intensity's coefficient (no rescaling needed)
+// A coefficient below the smallest normal number and those it is compared with, scaled by a power of two into range.
+template <class T>
+__device__ __forceinline__ void scale_small(T& I, T& Q, T& V) {
+    if (I >= smallest<T>()) return;
+    const T b = sizeof(T) == 4 ? T(18446744073709551616.0) : T(1.3407807929942597e154);   // 2^64, 2^512
+    I *= b; Q *= b; V *= b;
+}
+
+// cap_factor (coefficients.jl:264-288) from the ratios to the intensity's coefficient
 template <class T>
 __device__ __forceinline__ T row_cap(T I, T Q, T V) {
-    if (!(I >= smallest<T>())) return (Q == T(0) && V == T(0)) ? T(1) : T(0);
+    if (!(I > T(0))) return (Q == T(0) && V == T(0)) ? T(1) : T(0);
+    scale_small(I, Q, V);
     const T i = hrcp(I), q = Q * i, v = V * i, p2 = q * q + v * v;
     return p2 > T(0.9801) ? T(0.99) * hrsqrt(p2) : T(1);
 }
@@ -327,8 +336,8 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     const T ls = hlog2(nu * hrcp(nus)) * T(1.0 / 3);             // of the cube root of nu / nu_s
     const T c13 = hexp2(-ls), c23 = c13 * c13;
     const T e13 = hexp(T(-1.8899) * hexp2(ls));
-    constexpr double kJ = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);
-    const T iT = hrcp(Te), pj = T(kJ) * ne * nu * iT * iT * e13;
+    constexpr double kJ = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);   // times nu first: 2e-30 n_e underflows in FP32
+    const T iT = hrcp(Te), pj = T(kJ) * nu * ne * iT * iT * e13;
     const T jI = pj * T(2.5651) * (T(1) + T(1.92) * c13 + T(0.9977) * c23);
     const T jQ = pj * T(2.5651) * (T(1) + T(0.93193) * c13 + T(0.499873) * c23);
     const T jV = pj * T(4.0 / 3) * iT * ct * hrcp(st) * (T(1.81384) * nus * inu + T(3.42319) * c23 + T(0.0292545) * hexp2(T(-1.5) * ls) + T(2.03773) * c13);
