@@ -69,8 +69,7 @@ struct ks_context {
     int tune_nt = 0, tune_units = 0;        // the autotuner's choice for the mixed forward (0: the default)
     int nkv = 0;                            // knot values after the splat table in `tab`
     ks::TransportJob last_job{};            // the last forward pass with an adjoint's state
-    float* fwd_gstate = nullptr;            // set during the adjoint's forward pass only
-    unsigned char* fwd_gact = nullptr;
+    long long state_piece = 0;              // rays whose state the last gradient held at a time
     double adjoint_ms = 0.0;
     long long adjoint_launches = 0;
     bool count_events = false;
@@ -151,9 +150,12 @@ int launch_wind_stop(ks_context* c, int nmax, double slab);
 // FP64 throughout. The times, then the frequencies, lie in c->combos.
 int launch_mixed(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only);
 int launch_plain(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only);
-// The FP64 pass over the rays [j0, j0 + m) of a thermal scene with the reverse pass's state (for plain_state_rays rays).
-long long plain_state_rays(const ks_context* c, int nframes, int nfreq);
-int launch_plain_state(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m);
+// The pass over the rays [j0, j0 + m) of a thermal scene with the reverse pass's state, sized for `rays` rays: at most
+// state_rays. KS_ERR_OUT_OF_MEMORY: release_state, then again with a smaller_piece.
+long long state_rays(const ks_context* c, bool plain, int nframes, int nfreq);
+int launch_state(ks_context* c, bool plain, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long rays);
+void release_state(ks_context* c);
+long long smaller_piece(long long rays);
 
 // ---- the mixed reverse pass (ks_reverse.cu) --------------------------------------------------------------
 

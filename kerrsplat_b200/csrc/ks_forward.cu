@@ -47,20 +47,25 @@ static int stream_kernel(ks_context* c, long long j0, long long npix, long long 
     return KS_OK;
 }
 
-int launch_stream(ks_context* c) {
-    KS_CUDA(c, c->stream_buf.ensure(size_t(c->st.N) * SM_COUNT * c->npad * sizeof(float)));
+// ... of the rays [j0, j0 + m), npad apart
+static int mixed_stream(ks_context* c, long long j0, long long m, long long npad) {
+    KS_CUDA(c, c->stream_buf.ensure(size_t(c->st.N) * SM_COUNT * npad * sizeof(float)));
     float* out = c->stream_buf.as<float>();
-    return c->geo64 ? stream_kernel<double, float>(c, 0, c->npix, c->npad, out) : stream_kernel<float, float>(c, 0, c->npix, c->npad, out);
+    return c->geo64 ? stream_kernel<double, float>(c, j0, m, npad, out) : stream_kernel<float, float>(c, j0, m, npad, out);
 }
 
-int launch_wind_stop(ks_context* c, int nmax, double slab) {
+template <class T>
+static int wind_stop(ks_context* c, int nmax, double slab, long long j0, long long m, long long npad, const T* stream) {
     KS_CUDA(c, c->kstop.ensure(size_t(c->npix) * sizeof(int)));
-    k_wind_stop<float><<<nblocks(c->npix), kBlock, 0, c->stream>>>(plan_view(c), 0, c->npix, c->npad, c->stream_buf.as<float>(), nmax, float(slab),
-                                                                  c->kstop.as<int>());
+    k_wind_stop<T><<<nblocks(m), kBlock, 0, c->stream>>>(plan_view(c), j0, m, npad, stream, nmax, T(slab), c->kstop.as<int>());
     c->launches++;
     KS_CUDA(c, cudaGetLastError());
     return KS_OK;
 }
+
+int launch_stream(ks_context* c) { return mixed_stream(c, 0, c->npix, c->npad); }
+
+int launch_wind_stop(ks_context* c, int nmax, double slab) { return wind_stop(c, nmax, slab, 0, c->npix, c->npad, c->stream_buf.as<float>()); }
 
 // How a transport kernel of NT threads is shaped for a scene: samples per run, records per window, blocks per SM.
 struct Shape {
@@ -149,16 +154,18 @@ static TransportJob transport_job(ks_context* c, int ntot, int nframes, int nfre
     return job;
 }
 
+// The rays [j0, j0 + m), npad apart in the stream and the state (the reverse pass's, if there is one).
 template <int CH, int KM>
-static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab) {
+static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long npad,
+                    float* gstate, unsigned char* gact) {
     int nsm = 0;
     KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     // one march per ray, shared by every frame and frequency
-    int s = launch_stream(c);
-    if (s || (s = build_rows<float, KM>(c, ntot, c->fwd_gstate != nullptr))) return s;
-    TransportJob job = transport_job(c, ntot, nframes, nfreq, CH, L, 0, c->npix, c->npad);
+    int s = mixed_stream(c, j0, m, npad);
+    if (s || (s = build_rows<float, KM>(c, ntot, gstate != nullptr))) return s;
+    TransportJob job = transport_job(c, ntot, nframes, nfreq, CH, L, j0, m, npad);
     if (nmax >= 0) {
-        if ((s = launch_wind_stop(c, nmax, slab))) return s;
+        if ((s = wind_stop(c, nmax, slab, j0, m, npad, c->stream_buf.as<float>()))) return s;
         job.kstop = c->kstop.as<int>();
     }
     constexpr int B128 = 4, B256 = 2;
@@ -176,10 +183,10 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     // runs no longer than a segment
     if (wide) s256 = transport_shape<float, CH, KM, 256>(ntot, c->nkv, job.seg_len, B256);
     else s128 = transport_shape<float, CH, KM, 128>(ntot, c->nkv, job.seg_len, B128);
-    job.gstate = c->fwd_gstate;
-    job.gact = c->fwd_gact;
+    job.gstate = gstate;
+    job.gact = gact;
     c->last_job = job;   // as the reverse pass walks it
-    KS_CUDA(c, c->seg_out.ensure(size_t(nframes) * nfreq * job.nseg * c->npix * 20 * sizeof(float)));
+    KS_CUDA(c, c->seg_out.ensure(size_t(nframes) * nfreq * job.nseg * m * 20 * sizeof(float)));
     KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));   // the adjoint's two counters: no move under a captured render
     if (!c->capturing) cudaEventRecord(c->evc0, c->stream);
     s = wide ? run_transport<float, CH, KM, 256, B256>(c, job, s256, nsm, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix)
@@ -193,16 +200,18 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
 
 // Up to four frequencies share a unit's march, tests and frames.
 template <int KM>
-static int mixed_km(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab) {
-    if (nfreq >= 4) return mixed_ch<4, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    if (nfreq == 3) return mixed_ch<3, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    if (nfreq == 2) return mixed_ch<2, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
-    return mixed_ch<1, KM>(c, ntot, nframes, nfreq, L, nmax, slab);
+static int mixed_km(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long npad,
+                    float* gstate, unsigned char* gact) {
+    if (ntot > 32 * kMaxSplatWords) return fail(c, KS_ERR_ARGUMENT, "the mixed path takes at most %d splats (%d)", 32 * kMaxSplatWords, ntot);
+    if (nfreq >= 4) return mixed_ch<4, KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, npad, gstate, gact);
+    if (nfreq == 3) return mixed_ch<3, KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, npad, gstate, gact);
+    if (nfreq == 2) return mixed_ch<2, KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, npad, gstate, gact);
+    return mixed_ch<1, KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, npad, gstate, gact);
 }
 
 int launch_mixed(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only) {
-    if (ntot > 32 * kMaxSplatWords) return fail(c, KS_ERR_ARGUMENT, "the mixed path takes at most %d splats (%d)", 32 * kMaxSplatWords, ntot);
-    return thermal_only ? mixed_km<1>(c, ntot, nframes, nfreq, L, nmax, slab) : mixed_km<7>(c, ntot, nframes, nfreq, L, nmax, slab);
+    return thermal_only ? mixed_km<1>(c, ntot, nframes, nfreq, L, nmax, slab, 0, c->npix, c->npad, nullptr, nullptr)
+                        : mixed_km<7>(c, ntot, nframes, nfreq, L, nmax, slab, 0, c->npix, c->npad, nullptr, nullptr);
 }
 
 // FP64: the rays [j0, j0 + m), their stream and the transport over it; npad strides the stream and the state.
@@ -221,10 +230,8 @@ static int plain_piece(ks_context* c, int ntot, int nframes, int nfreq, double L
     }
     TransportJob job = transport_job(c, ntot, nframes, nfreq, 1, L, j0, m, npad);
     if (nmax >= 0) {
-        KS_CUDA(c, c->kstop.ensure(size_t(c->npix) * sizeof(int)));
-        k_wind_stop<double><<<nblocks(m), kBlock, 0, c->stream>>>(plan_view(c), j0, m, npad, stream, nmax, slab, c->kstop.as<int>());
-        c->launches++;
-        KS_CUDA(c, cudaGetLastError());
+        const int s = wind_stop(c, nmax, slab, j0, m, npad, stream);
+        if (s) return s;
         job.kstop = c->kstop.as<int>();
     }
     constexpr int B = 2;
@@ -244,33 +251,53 @@ static int clear_residuals(ks_context* c) {
     return KS_OK;
 }
 
-// The rays in pieces of at most 4 GB of stream.
+long long smaller_piece(long long rays) { return std::max<long long>(32, (rays / 2 + 31) / 32 * 32); }
+
+// The rays in pieces of at most 4 GB of stream and 4 GB of segment states (in one segment), halved until they fit.
 template <int KM>
 static int plain_km(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab) {
     int s = build_rows<double, KM>(c, ntot, false);
     if (s || (s = clear_residuals(c))) return s;
-    const size_t per_ray = size_t(c->st.N) * SM_COUNT * sizeof(double);
-    const long long piece = std::min<long long>(c->npad, std::max<long long>(32, (long long)((size_t(4) << 30) / per_ray) / 32 * 32));
-    for (long long j0 = 0; j0 < c->npix; j0 += piece)
-        if ((s = plain_piece<KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, c->npix - j0), piece, nullptr, nullptr))) return s;
+    const size_t per_ray = std::max(size_t(c->st.N) * SM_COUNT, size_t(nframes) * nfreq * 20) * sizeof(double);
+    long long piece = std::min<long long>(c->npad, std::max<long long>(32, (long long)((size_t(4) << 30) / per_ray) / 32 * 32));
+    for (long long j0 = 0; j0 < c->npix;) {
+        s = plain_piece<KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, c->npix - j0), piece, nullptr, nullptr);
+        if (s == KS_ERR_OUT_OF_MEMORY && piece > 32) {
+            cudaGetLastError();
+            c->stream64.release();
+            c->seg_out64.release();
+            piece = smaller_piece(piece);
+            j0 = 0;
+            continue;
+        }
+        if (s) return s;
+        j0 += piece;
+    }
     return KS_OK;
 }
 
-// Rays whose FP64 state (257 bytes a sample and combination) fits in 24 GB.
-long long plain_state_rays(const ks_context* c, int nframes, int nfreq) {
-    const size_t per_ray = size_t(nframes) * nfreq * c->st.N * (32 * sizeof(double) + 1);
+// Mixed: every ray. FP64: rays whose state (225 bytes a sample and combination) fits in 24 GB.
+long long state_rays(const ks_context* c, bool plain, int nframes, int nfreq) {
+    if (!plain) return c->npad;
+    const size_t per_ray = size_t(nframes) * nfreq * c->st.N * (kState * sizeof(double) + 1);
     return std::min<long long>(c->npad, std::max<long long>(32, (long long)((size_t(24) << 30) / per_ray) / 32 * 32));
 }
 
-int launch_plain_state(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m) {
-    int s = build_rows<double, 1>(c, ntot, true);
-    if (s || (j0 == 0 && (s = clear_residuals(c)))) return s;
-    const long long npad = plain_state_rays(c, nframes, nfreq);
-    const size_t rows = size_t(nframes) * nfreq * c->st.N * npad;
-    KS_CUDA(c, c->adj_state.ensure(rows * 32 * sizeof(double)));
+int launch_state(ks_context* c, bool plain, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long rays) {
+    const size_t rows = size_t(nframes) * nfreq * c->st.N * rays;
+    KS_CUDA(c, c->adj_state.ensure(rows * kState * (plain ? sizeof(double) : sizeof(float))));
     KS_CUDA(c, c->adj_act.ensure(rows));
     KS_CUDA(c, cudaMemsetAsync(c->adj_act.p, 0, rows, c->stream));
-    return plain_piece<1>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, npad, c->adj_state.as<double>(), c->adj_act.as<unsigned char>());
+    if (!plain)
+        return mixed_km<1>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, rays, c->adj_state.as<float>(), c->adj_act.as<unsigned char>());
+    int s = build_rows<double, 1>(c, ntot, true);
+    if (s || (j0 == 0 && (s = clear_residuals(c)))) return s;
+    return plain_piece<1>(c, ntot, nframes, nfreq, L, nmax, slab, j0, m, rays, c->adj_state.as<double>(), c->adj_act.as<unsigned char>());
+}
+
+void release_state(ks_context* c) {
+    cudaGetLastError();
+    for (DevBuf* d : {&c->adj_state, &c->adj_act, &c->adj_bnd, &c->adj_unit, &c->adj_part, &c->stream64, &c->seg_out64, &c->seg_out}) d->release();
 }
 
 int launch_plain(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, bool thermal_only) {

@@ -1615,8 +1615,44 @@ int stage_dev(ks_context* c, DevBuf& buf, const U* src, size_t count, const U** 
     return s;
 }
 
-// The forward image with the state the reverse pass needs (FP64: stored samples, cutoffs, tails),
-// the seeds (given, or those of chi^2), the reverse pass and the reduction into dparams.
+// The forward and the reverse pass of a gradient, the state of `piece` rays at a time. With the state of every ray held,
+// the forward pass leaves it; else the forward pass is the image alone and the reverse pass goes over the screen piece by
+// piece. Pieces are halved while memory runs out (`fixed`: not in a capture, which takes the piece of the call before it).
+struct GradientPasses {
+    ks_context* c;
+    int ntot, nframes, nfreq, nmax;
+    double L, slab;
+    bool plain, fixed;
+    long long piece;
+    bool shrink(int s) {
+        if (s != KS_ERR_OUT_OF_MEMORY || fixed || piece <= 32) return false;
+        release_state(c);
+        piece = smaller_piece(piece);
+        return true;
+    }
+    int state(long long j0) { return launch_state(c, plain, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, c->npix - j0), piece); }
+    int forward() {
+        int s = KS_OK;
+        do
+            s = piece >= c->npix ? state(0) : plain ? launch_plain(c, ntot, nframes, nfreq, L, nmax, slab, true)
+                                                    : launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, true);
+        while (shrink(s));
+        return s;
+    }
+    int reverse() {
+        for (long long j0 = 0; ntot > 0 && j0 < c->npix;) {
+            int s = piece < c->npix ? state(j0) : KS_OK;
+            if (s == KS_OK) s = launch_reverse(c, ntot, nmax, plain, j0 > 0);
+            if (shrink(s)) { j0 = 0; continue; }
+            if (s) return s;
+            j0 += piece;
+        }
+        c->state_piece = piece;
+        return KS_OK;
+    }
+};
+
+// The forward image, the seeds (given, or those of chi^2), the reverse pass and the reduction into dparams.
 int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double* times, int nframes, const double* nus, int nfreq,
                 double L, int precision, int nmax, double slab, const double* dstokes, int order, const double* data,
                 const double* sigma, double sigma_s, const uint8_t* mask, double* chi2_out, double* dparams, int accumulate,
@@ -1658,25 +1694,10 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
     cudaEventRecord(c->ev0, c->stream);
     const bool mixed = precision == KS_MIXED;
     // 1. forward pass with the reverse pass's state
-    const long long piece = mixed ? n : plain_state_rays(c, nframes, nfreq);   // FP64: rays whose state is held at a time
-    if (mixed) {
-        c->geo64 = geo;
-        const size_t rows = size_t(ncombo) * N * c->npad;
-        KS_CUDA(c, c->adj_state.ensure(rows * 32 * sizeof(float)));
-        KS_CUDA(c, c->adj_act.ensure(rows));
-        KS_CUDA(c, cudaMemsetAsync(c->adj_act.p, 0, rows, c->stream));
-        c->fwd_gstate = c->adj_state.as<float>();
-        c->fwd_gact = c->adj_act.as<unsigned char>();
-        int s = launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, true);
-        c->fwd_gstate = nullptr;
-        c->fwd_gact = nullptr;
-        if (s) return s;
-    } else {
-        if (size_t(ntot) * ST_COUNT * sizeof(double) > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for the FP64 adjoint (%d)", ntot);
-        int s = piece >= n ? launch_plain_state(c, ntot, nframes, nfreq, L, nmax, slab, 0, n)
-                           : launch_plain(c, ntot, nframes, nfreq, L, nmax, slab, true);
-        if (s) return s;
-    }
+    if (mixed) c->geo64 = geo;
+    else if (size_t(ntot) * ST_COUNT * sizeof(double) > 200 * 1024) return fail(c, KS_ERR_ARGUMENT, "too many splats for the FP64 adjoint (%d)", ntot);
+    GradientPasses passes{c, ntot, nframes, nfreq, nmax, L, slab, !mixed, false, state_rays(c, !mixed, nframes, nfreq)};
+    if (int s = passes.forward()) return s;
     // 2. seeds
     const long long nblk = (nrc + 255) / 256;
     double vis_chi2 = 0.0;
@@ -1747,17 +1768,7 @@ int adjoint_run(ks_context* c, const ks_splat_set* sets, int nsets, const double
         KS_CUDA(c, cudaGetLastError());
     }
     // 3. reverse pass and the deterministic reduction
-    if (ntot > 0 && mixed) {
-        int s = launch_reverse(c, ntot, nmax, false, false);
-        if (s) return s;
-    } else if (ntot > 0) {
-        for (long long j0 = 0; j0 < n; j0 += piece) {
-            int s = KS_OK;
-            if (piece < n) s = launch_plain_state(c, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, n - j0));
-            if (s == KS_OK) s = launch_reverse(c, ntot, nmax, true, j0 > 0);
-            if (s) return s;
-        }
-    }
+    if (int s = passes.reverse()) return s;
     cudaEventRecord(c->ev1, c->stream);
     // 4. results; the gradient only if no kernel gave up
     const long long ng = (long long)ntot * GR_COUNT;
@@ -1837,30 +1848,21 @@ int ks_chi2_gradient_graph_capture(ks_context* c, const ks_splat_set* sets, int3
     const int ncombo = nframes * nfreq;
     const long long nrc = n * ncombo;
     const long long nblk = (nrc + 255) / 256;
-    const size_t rows = size_t(ncombo) * c->st.N * c->npad;
     if ((status = copy_graph_inputs(c, c->cgraph_tab, c->cgraph_combos, ntot, nframes, nfreq))) return status;
     GraphInputs own(c, c->cgraph_tab, c->cgraph_combos);
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     c->capturing = true;
     status = capture_tables(c, sets, nsets, ntot, true);
-    if (status == KS_OK && ntot > 0) {
-        // the forward pass with the reverse pass's state
-        c->geo64 = false;
-        if (cudaMemsetAsync(c->adj_act.p, 0, rows, c->stream) != cudaSuccess) status = fail(c, KS_ERR_DEVICE, "graph capture: activity reset");
-        c->fwd_gstate = c->adj_state.as<float>();
-        c->fwd_gact = c->adj_act.as<unsigned char>();
-        if (status == KS_OK) status = launch_mixed(c, ntot, nframes, nfreq, L, nmax, slab, true);
-        c->fwd_gstate = nullptr;
-        c->fwd_gact = nullptr;
-    }
+    c->geo64 = false;
+    GradientPasses passes{c, ntot, nframes, nfreq, nmax, L, slab, false, true, c->state_piece};
+    if (status == KS_OK) status = passes.forward();
     if (status == KS_OK) {
         k_chi2_seed<<<unsigned(nblk), 256, 0, c->stream>>>(c->out_sorted.as<double>(), c->perm.as<long long>(), n, ncombo, data, sigma,
                                                            sigma_scalar, mask, c->seeds.as<double>(), c->chi_part.as<double>());
         k_sum_partials<<<1, 256, 0, c->stream>>>(c->chi_part.as<double>(), nblk, c->chi_val.as<double>());
         if (cudaGetLastError() != cudaSuccess) status = fail(c, KS_ERR_DEVICE, "graph capture: chi^2 seeds");
     }
-    if (status == KS_OK && ntot > 0)
-        status = launch_reverse(c, ntot, nmax, false, false);
+    if (status == KS_OK) status = passes.reverse();
     const long long ng = (long long)ntot * GR_COUNT;
     if (status == KS_OK && ng > 0) {
         k_accumulate<<<nblocks(ng, 256), 256, 0, c->stream>>>(dparams, c->dgrad.as<double>(), ng, accumulate, c->errflag.as<unsigned>());
@@ -1924,8 +1926,14 @@ int jvp_chunk(ks_context* c, int ntot, const double* dparams_dev, const double* 
         // segments until there are some 32 warps per SM (at least 16 samples each), as far as 4 GB of segment states go
         int nseg = 1;
         while (nrc * nseg < 148LL * 1024 && (nseg * 2) * 16 <= c->st.N && nrc * nseg * 2 * 20 * (K + 1) * (long long)sizeof(float) <= (4LL << 30)) nseg *= 2;
+        // fewer where memory runs out
+        for (;; nseg /= 2) {
+            const cudaError_t e = c->jvp_part.ensure(size_t(nrc) * nseg * 20 * (K + 1) * sizeof(float));
+            if (e == cudaErrorMemoryAllocation && nseg > 1) { cudaGetLastError(); continue; }
+            KS_CUDA(c, e);
+            break;
+        }
         const int seg_len = (c->st.N + nseg - 1) / nseg;
-        KS_CUDA(c, c->jvp_part.ensure(size_t(nrc) * nseg * 20 * (K + 1) * sizeof(float)));
         const int* kstop = nullptr;
         if (nmax >= 0) {
             int s = launch_wind_stop(c, nmax, slab);

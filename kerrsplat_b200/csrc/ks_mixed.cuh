@@ -213,6 +213,9 @@ k_stream_block(PlanView P, Spacetime st, long long j0, long long npix, long long
     }
 }
 
+// The adjoint's state of a sample: P before it (16), the coefficients (11), the step length: whole 16-byte words.
+constexpr int kState = 28;
+
 // A transport pass and its segmentation, as the reverse pass walks it too: work units of 32 consecutive sorted rays x
 // one segment of the sample range x one frame x up to `ch` frequencies, the last rays first (the plunging rays
 // near the centre of the screen, sorted last, carry most of the work).
@@ -221,7 +224,7 @@ struct TransportJob {
     int nframes, nfreq, nseg, seg_len, nvc;
     long long nchunks;               // 32-ray groups
     double L;
-    void* gstate = nullptr;          // the adjoint's state: 32 values of T per (combination, sample, ray): P before the sample, the coefficients, the step length
+    void* gstate = nullptr;          // the adjoint's state: kState values of T per (combination, sample, ray)
     unsigned char* gact = nullptr;   // and 1 where the sample has a step
     const int* kstop = nullptr;      // the first sample beyond the half-orbit cutoff (null: none)
     int ntot = 0, nkv = 0, run = 64, cap = 0, rows_shared = 1;

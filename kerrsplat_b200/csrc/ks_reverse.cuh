@@ -506,7 +506,7 @@ k_reverse(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ rows
                     if (!((actb[at] >> c) & 1u)) { rp[14] = T(0); continue; }
                     const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + (at >> 5) - 1)) * npad + jb + (at & 31);
                     T v[kRec], w[kRec];
-                    get16<12>(gstate + g * 32 + 16, v);
+                    get16<12>(gstate + g * kState + 16, v);
                     step_record(c_moments, v, v[11], w);
                     put16<kRec>(rp, w);
                 }
@@ -541,8 +541,8 @@ k_reverse(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ rows
                     if (rp[14] == T(0)) continue;
                     const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + (at >> 5) - 1)) * npad + jb + o;
                     T Pm[16], in[12], wk[4], Rt[4], O[16], E[4], cb[12];
-                    get16<16>(gstate + g * 32, Pm);
-                    get16<12>(gstate + g * 32 + 16, in);
+                    get16<16>(gstate + g * kState, Pm);
+                    get16<12>(gstate + g * kState + 16, in);
                     get16<4>(rp + 4, Rt);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)

@@ -971,7 +971,7 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                     if (gstate) {
                         const int at = order2[id];
                         const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + (at >> 5) - 1)) * npad + jb + (at & 31);
-                        put16<12>(gstate + g * 32 + 16, v);
+                        put16<12>(gstate + g * kState + 16, v);
                         job.gact[g] = 1;
                     }
                     T w[kRec];
@@ -993,7 +993,7 @@ k_transport(PlanView P, Spacetime st, TransportJob job, const T* __restrict__ ro
                         if (v[14] == T(0)) continue;
                         if (gstate) {
                             const long long g = (((long long)(v0 + c) * job.nframes + f) * N + (kr + kl - 1)) * npad + jb + lane;
-                            put16<4>(gstate + g * 32 + 4 * row, pr[q]);
+                            put16<4>(gstate + g * kState + 4 * row, pr[q]);
                         }
                         T p1[4], p2[4], p3[4];
                         kvec_t(v + 8, pr[q], p1); kvec_t(v + 8, p1, p2); kvec_t(v + 8, p2, p3);

@@ -201,3 +201,41 @@ def test_fp32_thin_plasma(ln_ne):
     g = ks.adjoint(cache, m, [0.0], [230e9], L, ds)
     assert rel(ks.adjoint(cache, m, [0.0], [230e9], L, ds, precision=ks.KS_MIXED), g) < 1e-3
     cache.close()
+
+
+@pytest.mark.parametrize("precision", [ks.KS_FP64, ks.KS_MIXED])
+def test_gradients_and_renders_in_little_memory(precision):
+    """With 600 MB of the device free, less than the state of every ray (1.9 GB in FP64, 0.95 GB in FP32), the gradient,
+    its captured graph and the FP64 stream (0.54 GB beside other buffers) go over the screen in pieces. The sums are the
+    same but for their grouping: 1e-11 in FP64, 1e-5 in FP32."""
+    import torch
+    rng = np.random.Generator(np.random.PCG64(30))
+    m = ks.PolarizedSplats(torch.tensor(scenes.thermal_params(rng, 10, A, rlo=3.0, rhi=8.0), device="cuda"))
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), 128)
+    data = torch.tensor(rng.standard_normal((1, 1, cam.npix, 4)) * 1e-6, device="cuda")
+
+    def calls():
+        cache = ks.regenerate(ks.GeodesicCache(cam, 512), A, THO)
+        chi2, g, img = ks.chi2_gradient(cache, m, [0.0], [230e9], L, data, 1e-7, precision=precision, return_image=True)
+        out = [chi2, np.asarray(g), np.asarray(img.cpu()), np.asarray(ks.render(cache, m, [0.0], [230e9], L, precision=precision).cpu())]
+        if precision == ks.KS_MIXED:
+            graph = ks.capture_chi2_gradient(cache, m, [0.0], [230e9], L, data, 1e-7)
+            graph.dparams.zero_()
+            out.append(graph.replay()[1].cpu().numpy().reshape(10, 21).T)
+        cache.close()
+        return out
+
+    want = calls()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    held = torch.empty(free - 600 * 2 ** 20, dtype=torch.uint8, device="cuda")
+    try:
+        got = calls()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    tol = 1e-11 if precision == ks.KS_FP64 else 1e-5
+    for x, y in zip(got, want):
+        assert np.all(np.isfinite(x)) and rel(x, y) < tol
+    if precision == ks.KS_MIXED:
+        assert rel(got[4], got[1]) < 1e-12
