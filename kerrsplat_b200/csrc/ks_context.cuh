@@ -103,6 +103,7 @@ inline int fail(ks_context* c, int code, const char* fmt, ...) {
 }
 
 inline int cuda_fail(ks_context* c, cudaError_t e, const char* what) {
+    cudaGetLastError();   // reported here: the next call (of any context) checks its own launches
     if (e == cudaErrorMemoryAllocation) return fail(c, KS_ERR_OUT_OF_MEMORY, "%s: %s", what, cudaGetErrorString(e));
     return fail(c, KS_ERR_DEVICE, "%s: %s", what, cudaGetErrorString(e));
 }

@@ -263,7 +263,6 @@ static int plain_km(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     for (long long j0 = 0; j0 < c->npix;) {
         s = plain_piece<KM>(c, ntot, nframes, nfreq, L, nmax, slab, j0, std::min(piece, c->npix - j0), piece, nullptr, nullptr);
         if (s == KS_ERR_OUT_OF_MEMORY && piece > 32) {
-            cudaGetLastError();
             c->stream64.release();
             c->seg_out64.release();
             piece = smaller_piece(piece);
@@ -296,7 +295,6 @@ int launch_state(ks_context* c, bool plain, int ntot, int nframes, int nfreq, do
 }
 
 void release_state(ks_context* c) {
-    cudaGetLastError();
     for (DevBuf* d : {&c->adj_state, &c->adj_act, &c->adj_bnd, &c->adj_unit, &c->adj_part, &c->stream64, &c->seg_out64, &c->seg_out}) d->release();
 }
 

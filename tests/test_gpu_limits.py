@@ -239,3 +239,26 @@ def test_gradients_and_renders_in_little_memory(precision):
         assert np.all(np.isfinite(x)) and rel(x, y) < tol
     if precision == ks.KS_MIXED:
         assert rel(got[4], got[1]) < 1e-12
+
+
+def test_a_failed_allocation_is_over_with_its_call():
+    """A call that finds no memory raises MemoryError, and the calls after it, on this context and on a new one, run."""
+    import torch
+    m = ks.PolarizedSplats(wide_splats(3, 31))
+    cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), 96)
+    cache = ks.regenerate(ks.GeodesicCache(cam, 1024), A, THO)
+    small = cache_of(7, 6, 32)
+    want = np.asarray(ks.render(small, m, [0.0], [230e9], L, precision=ks.KS_MIXED))
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - 200 * 2 ** 20, dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(MemoryError):
+            ks.render(cache, m, [0.0], [230e9], L, precision=ks.KS_MIXED)   # a stream of 0.3 GB
+        assert np.array_equal(ks.render(small, m, [0.0], [230e9], L, precision=ks.KS_MIXED), want)
+        cache_of(5, 4, 16).close()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert np.abs(np.asarray(ks.render(cache, m, [0.0], [230e9], L, precision=ks.KS_MIXED))).max() > 0
+    cache.close()
+    small.close()
