@@ -46,14 +46,13 @@ struct ks_context {
     DevBuf alpha, beta, key, key2, idx, perm, plan, nanch, aoff, anchors, resid_t, resid_phi, scratch;
     DevBuf tab, combos, out_sorted, stage_in, stage_out, counters, seg_out, work, stream_buf;
     DevBuf inv_perm, dft_tu, dft_tv, dft_a, dft_t, dft_c, dft_s, dft_in[8], dft_partial;
-    // adjoint: gradient table, stored FP64 samples (plain path), cutoffs, tails, per-ray slots,
-    // seeds, chi^2 partials; mixed path: per-sample states, activity, segment bounds, unit partials
-    DevBuf gtab, samples, kstop, dgrad, seeds, chi_part, chi_val, dstage;
+    // adjoint: gradient table, cutoffs, the gradient, seeds, chi^2 partials; per-sample states, activity, segment bounds,
+    // unit partials
+    DevBuf gtab, kstop, dgrad, seeds, chi_part, chi_val, dstage;
     DevBuf adj_state, adj_act, adj_bnd, adj_unit, adj_part, jvp_tab, jvp_in, jvp_out, jvp_part, st_buf;
     DevBuf rows;      // the transport's splat rows and knot array (FP32 or FP64)
     DevBuf thin_part;             // the thin image's pieces (sized by regenerate)
     DevBuf stream64, seg_out64;   // the FP64 render's stream and segment states
-    DevBuf tab32;     // the splat table and knot array in FP32, padded to 16 bytes (the TMA staging source)
     DevBuf errflag;   // set by a kernel whose bounded wait gave up
     cudaGraph_t graph = nullptr;          // ks_render_graph_capture: one mixed render of device-resident sets
     cudaGraphExec_t graph_exec = nullptr;

@@ -339,12 +339,6 @@ __global__ void k_anchor_prefix(long long npix, long long npad, const double* __
 
 // ---- kernels: splat tables ---------------------------------------------------------------------------
 
-// the table (and knot array) in FP32 for the mixed kernels' staging copy, zero-padded to np4 floats
-__global__ void k_tab_f32(long long n, long long np4, const double* __restrict__ src, float* __restrict__ dst) {
-    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q < np4) dst[q] = q < n ? float(src[q]) : 0.f;
-}
-
 // K0 and K1 from K_nu(x) = int_0^inf exp(-x cosh t) cosh(nu t) dt by the trapezoidal rule.
 __host__ __device__ void besselk01(double x, double& k0, double& k1) {
     // trapezoid in t on exp(-x (cosh t - 1)) (the factor exp(-x) applied at the end); the step
@@ -913,15 +907,6 @@ int build_tables(ks_context* c, const ks_splat_set* sets, int nsets, int* ntot_o
         tmp.release();
         first += S.nsplat;
     }
-    // the FP32 copy the mixed kernels stage into shared memory (a multiple of 16 bytes)
-    {
-        const long long nv = (long long)ntot * ST_COUNT + c->nkv;
-        const long long np4 = std::max<long long>(4, (nv + 3) / 4 * 4);
-        KS_CUDA(c, c->tab32.ensure(size_t(np4) * sizeof(float)));
-        k_tab_f32<<<nblocks(np4, 256), 256, 0, c->stream>>>(nv, np4, c->tab.as<double>(), c->tab32.as<float>());
-        c->launches++;
-        KS_CUDA(c, cudaGetLastError());
-    }
     *ntot_out = ntot;
     return KS_OK;
 }
@@ -1433,8 +1418,8 @@ int ks_riaf_image(ks_context* c, const double* model, int32_t pandya, const doub
 
 // The device buffers a captured render reads or writes (a replay requires them unmoved).
 std::vector<void*> graph_buffers(const ks_context* c) {
-    return {c->tab32.p, c->rows.p, c->kstop.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->errflag.p, c->perm.p,
-            c->plan.p, c->anchors.p, c->aoff.p};
+    return {c->rows.p, c->kstop.p, c->stream_buf.p, c->seg_out.p, c->work.p, c->out_sorted.p, c->errflag.p, c->perm.p, c->plan.p,
+            c->anchors.p, c->aoff.p};
 }
 
 void release_graph(cudaGraph_t& g, cudaGraphExec_t& ex) {
@@ -1472,7 +1457,7 @@ int copy_graph_inputs(ks_context* c, DevBuf& tab, DevBuf& combos, int ntot, int 
 
 // The splat tables of device-resident sets rebuilt on the device inside a capture (the knot array
 // stays as the ordinary call before the capture wrote it): k_splat_table per set, with grad the
-// gradient table (k_grad_table), and the FP32 copy.
+// gradient table (k_grad_table).
 int capture_tables(ks_context* c, const ks_splat_set* sets, int nsets, int ntot, bool grad) {
     int first = 0, koff = 0;
     for (int s = 0; s < nsets; ++s) {
@@ -1490,15 +1475,11 @@ int capture_tables(ks_context* c, const ks_splat_set* sets, int nsets, int ntot,
         first += S.nsplat;
         koff += S.nsplat * 4 * nk;   // per knot splat: its nk times and 3 nk centres
     }
-    const long long nv = (long long)ntot * ST_COUNT + c->nkv;
-    const long long np4 = std::max<long long>(4, (nv + 3) / 4 * 4);
-    k_tab_f32<<<nblocks(np4, 256), 256, 0, c->stream>>>(nv, np4, c->tab.as<double>(), c->tab32.as<float>());
-    if (cudaGetLastError() != cudaSuccess) return fail(c, KS_ERR_DEVICE, "graph capture: FP32 table");
     return KS_OK;
 }
 
 // One mixed render of device-resident splat sets recorded into a CUDA graph: the splat tables built
-// from the parameters (in place on the device), their FP32 copy, the sample stream, the consumer, the
+// from the parameters (in place on the device), the sample stream, the transport, the
 // segment composition and the output in `order`. Frames, frequencies, L, the knot array, the splat
 // counts and the pointers are fixed at capture; a replay re-reads the parameter values.
 int ks_render_graph_capture(ks_context* c, const ks_splat_set* sets, int32_t nsets, const double* times, int32_t nframes,

@@ -318,17 +318,6 @@ __device__ __forceinline__ Coef<T> kappa_cs(T ne, T kap, T w, T hyp, T g43, T g2
     return {jI, jQ, jV, aI, aQ, aV, rQ, rV};
 }
 
-// The fits at the pitch angle th (the reference's signatures): its sine and cosine.
-template <class T>
-__device__ __forceinline__ Coef<T> thermal(T ne, T Te, T f0, T kr, T B, T nu, T th) { return thermal_cs(ne, Te, f0, kr, B, nu, sin(th), cos(th)); }
-template <class T>
-__device__ __forceinline__ Coef<T> powerlaw(T ne, T p, T gmin, T gspan, T gamj, T gama, T B, T nu, T th) {
-    return powerlaw_cs(ne, p, gmin, gspan, gamj, gama, B, nu, sin(th), cos(th));
-}
-template <class T>
-__device__ __forceinline__ Coef<T> kappa(T ne, T kap, T w, T hyp, T g43, T g2, T gq, T gp, T gk2, T kb, T B, T nu, T th) {
-    return kappa_cs(ne, kap, w, hyp, g43, g2, gq, gp, gk2, kb, B, nu, sin(th), cos(th));
-}
 // The pitch angle's sine and cosine from its (clamped) cosine: sin(acos c) = sqrt((1 - c)(1 + c)).
 template <class T>
 __device__ __forceinline__ void pitch_sc(T cosB, T& st, T& ct) {
@@ -789,38 +778,6 @@ __device__ __forceinline__ void kmul_t(const T K[16], const T v[4], T out[4]) {
 }
 template <class T>
 __device__ __forceinline__ T dot4(const T x[4], const T y[4]) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3]; }
-
-// The exact step in its structured form: O = sum_n o_n K^n, E = s sum_n e_n K^n j with the
-// coefficients of step_coefficients, K the rescaled matrix and s the power-of-two rescaling: the same
-// operator as transfer_step (the same branches and thresholds), with one assembly for all branches.
-template <class T>
-__device__ __forceinline__ void transfer_step_structured(const MomentCoeffs& MC, const T j4[4], const T al[4], const T rh[3], T Dl, T O[16],
-                                                         T E[4]) {
-    const T s = pow2_below(Dl);
-    const T D = Dl / s;
-    const T aI = al[0] * s, aQ = al[1] * s, aU = al[2] * s, aV = al[3] * s, rQ = rh[0] * s, rU = rh[1] * s, rV = rh[2] * s;
-    T o[4], e[4];
-    step_coefficients(MC, aI * D, aQ * aQ + aU * aU + aV * aV, rQ * rQ + rU * rU + rV * rV, aQ * rQ + aU * rU + aV * rV, D, o, e);
-    T K[16];
-    K[0] = 0; K[1] = aQ; K[2] = aU; K[3] = aV; K[4] = aQ; K[5] = 0; K[6] = rV; K[7] = -rU;
-    K[8] = aU; K[9] = -rV; K[10] = 0; K[11] = rQ; K[12] = aV; K[13] = rU; K[14] = -rQ; K[15] = 0;
-    T K2[16];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) K2[4 * i + jj] = K[4 * i] * K[jj] + K[4 * i + 1] * K[4 + jj] + K[4 * i + 2] * K[8 + jj] + K[4 * i + 3] * K[12 + jj];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const T k3 = K2[4 * i] * K[jj] + K2[4 * i + 1] * K[4 + jj] + K2[4 * i + 2] * K[8 + jj] + K2[4 * i + 3] * K[12 + jj];
-            O[4 * i + jj] = ((i == jj) ? o[0] : T(0)) + o[1] * K[4 * i + jj] + o[2] * K2[4 * i + jj] + o[3] * k3;
-        }
-    T Kj[4], K2j[4], K3j[4];
-    kmul(K, j4, Kj); kmul(K, Kj, K2j); kmul(K, K2j, K3j);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) E[i] = s * (e[0] * j4[i] + e[1] * Kj[i] + e[2] * K2j[i] + e[3] * K3j[i]);
-}
 
 // ---- coordinates ------------------------------------------------------------------------------------
 

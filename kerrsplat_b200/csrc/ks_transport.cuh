@@ -551,7 +551,7 @@ __device__ __forceinline__ void step_scalars(const MomentCoeffs& MC, T a, T a2, 
     e[3] = (Is - Ish) * iTh;
 }
 
-// A step record: o_0..3, E, the six entries of the rescaled K, the active flag (transfer_step_structured
+// A step record: o_0..3, E, the six entries of the rescaled K, the active flag (transfer_step
 // without its matrices).
 constexpr int kRec = 16;
 template <class T>
