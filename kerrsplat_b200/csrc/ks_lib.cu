@@ -1006,8 +1006,10 @@ int ks_context_destroy(ks_context* c) {
     if (c->evg0) cudaEventDestroy(c->evg0);
     if (c->evg1) cudaEventDestroy(c->evg1);
     if (c->ev1) cudaEventDestroy(c->ev1);
-    if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-    if (c->graph) cudaGraphDestroy(c->graph);
+    for (cudaGraphExec_t g : {c->graph_exec, c->cgraph_exec})
+        if (g) cudaGraphExecDestroy(g);
+    for (cudaGraph_t g : {c->graph, c->cgraph})
+        if (g) cudaGraphDestroy(g);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return KS_OK;

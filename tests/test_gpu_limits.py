@@ -304,3 +304,23 @@ def test_both_sides_of_the_block_march(precision, rays, tol):
         cache.close()
     assert np.abs(out[0]).max() > 0
     assert rel(out[0], out[1]) < tol
+
+
+def test_a_closed_context_leaves_no_graph():
+    """Contexts closed with both their graphs captured give all of the device's memory back (a graph holds some 150 KB)."""
+    import torch
+    m = ks.PolarizedSplats(torch.tensor(wide_splats(3, 36), device="cuda"))
+
+    def one():
+        cache = cache_of(9, 7, 32)
+        data = torch.zeros((1, 1, cache.npix, 4), dtype=torch.float64, device="cuda")
+        ks.capture_render(cache, m, [0.0], [230e9], L).replay()
+        ks.capture_chi2_gradient(cache, m, [0.0], [230e9], L, data, 1e-6).replay()
+        cache.close()
+
+    for _ in range(3):
+        one()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(60):
+        one()
+    assert before - torch.cuda.mem_get_info()[0] <= 4 * 2 ** 20
