@@ -357,6 +357,7 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
 
 // The power-law and kappa fits (powerlaw_cs, kappa_cs) from the row's constants, out of line: scenes that mix
 // populations run them a population at a time. As there, a field along the ray is evaluated 1e-6 from the axis.
+// lo: the low limit times its scale (n_e and nu_c first: the limit alone times the power underflows in FP32 at large kappa)
 template <class T>
 __device__ __forceinline__ T kappa_bridge(T lo, T arg, T ix) { return lo * hexp2(-ix * hlog2(T(1) + hexp2(arg))); }
 
@@ -382,10 +383,10 @@ __device__ __noinline__ bool other_row(const T* r, int kind, T ne, T nu, T st, T
     } else {
         const T X = nu * hrcp(nb) * e[EK_X], lx = hlog2(X);
         const T pj = ne * nb * hexp2(T(1.0 / 3) * lx), pa = ne * hrcp(nb) * hexp2(T(-5.0 / 3) * lx);
-        jI = pj * kappa_bridge(e[EK_I], e[EK_I + 1] * lx + e[EK_I + 2], e[EK_I + 3]);
-        jQ = pj * kappa_bridge(e[EK_Q], e[EK_Q + 1] * lx + e[EK_Q + 2], e[EK_Q + 3]);
-        aI = pa * kappa_bridge(e[EK_AI], e[EK_AI + 1] * lx + e[EK_AI + 2], e[EK_AI + 3]);
-        aQ = pa * kappa_bridge(e[EK_AQ], e[EK_AQ + 1] * lx + e[EK_AQ + 2], e[EK_AQ + 3]);
+        jI = kappa_bridge(pj * e[EK_I], e[EK_I + 1] * lx + e[EK_I + 2], e[EK_I + 3]);
+        jQ = kappa_bridge(pj * e[EK_Q], e[EK_Q + 1] * lx + e[EK_Q + 2], e[EK_Q + 3]);
+        aI = kappa_bridge(pa * e[EK_AI], e[EK_AI + 1] * lx + e[EK_AI + 2], e[EK_AI + 3]);
+        aQ = kappa_bridge(pa * e[EK_AQ], e[EK_AQ + 1] * lx + e[EK_AQ + 2], e[EK_AQ + 3]);
         // circular: the limits carry (sin^-u - 1)^v and X^-0.35 against X^-0.5
         const T u1 = hexp2(T(-12.0 / 5) * ls) - T(1), u2 = hexp2(T(-2.5) * ls) - T(1);
         const T u3 = hexp2(T(-114.0 / 50) * ls) - T(1), u4 = hexp2(T(-41.0 / 20) * ls) - T(1);
@@ -393,11 +394,11 @@ __device__ __noinline__ bool other_row(const T* r, int kind, T ne, T nu, T st, T
         jV = aV = T(0);
         if (u1 > T(0) && u2 > T(0)) {
             const T l1 = T(12.0 / 25) * hlog2(u1), l2 = T(11.0 / 25) * hlog2(u2);
-            jV = sg * pj * x35 * kappa_bridge(e[EK_V] * hexp2(l1), e[EK_V + 3] * (e[EK_V + 1] * lx + e[EK_V + 2] + l1 - l2 + T(3.0 / 20) * lx), e[EK_V + 4]);
+            jV = sg * kappa_bridge(pj * x35 * e[EK_V] * hexp2(l1), e[EK_V + 3] * (e[EK_V + 1] * lx + e[EK_V + 2] + l1 - l2 + T(3.0 / 20) * lx), e[EK_V + 4]);
         }
         if (u3 > T(0) && u4 > T(0)) {
             const T l3 = T(223.0 / 500) * hlog2(u3), l4 = T(0.5) * hlog2(u4);
-            aV = sg * pa * x35 * kappa_bridge(e[EK_AV] * hexp2(l3), e[EK_AV + 3] * (e[EK_AV + 1] * lx + e[EK_AV + 2] + l3 - l4 + T(3.0 / 20) * lx), e[EK_AV + 4]);
+            aV = sg * kappa_bridge(pa * x35 * e[EK_AV] * hexp2(l3), e[EK_AV + 3] * (e[EK_AV + 1] * lx + e[EK_AV + 2] + l3 - l4 + T(3.0 / 20) * lx), e[EK_AV + 4]);
         }
         const int i = int(e[EK_FIT]);
         auto fit_q = [&](int n) {

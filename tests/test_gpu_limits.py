@@ -324,3 +324,18 @@ def test_a_closed_context_leaves_no_graph():
     for _ in range(60):
         one()
     assert before - torch.cuda.mem_get_info()[0] <= 4 * 2 ** 20
+
+
+@pytest.mark.parametrize("kappa", [3.05, 7.0, 12.0, 25.0])
+def test_fp32_steep_kappa_distributions(kappa):
+    """Kappa splats so steep that their image is 1e-20 of an ordinary one's (1e-26): the FP32 image is within 1e-4 of
+    FP64, its budget."""
+    rng = np.random.Generator(np.random.PCG64(35))
+    p = scenes.kappa_params(rng, 4, A)
+    p[3:6] = np.log(rng.uniform(0.8, 2.0, (3, 4)))
+    p[13], p[14] = kappa, -2.0
+    cache, m = cache_of(9, 7, 70), ks.KappaSplats(p)
+    img = np.asarray(ks.render(cache, m, [0.0], [230e9], L))
+    assert np.all(np.isfinite(img)) and np.abs(img).max() > 0
+    assert rel(ks.render(cache, m, [0.0], [230e9], L, precision=ks.KS_MIXED), img) < 1e-4
+    cache.close()
