@@ -307,7 +307,8 @@ def test_both_sides_of_the_block_march(precision, rays, tol):
 
 
 def test_a_closed_context_leaves_no_graph():
-    """Contexts closed with both their graphs captured give all of the device's memory back (a graph holds some 150 KB)."""
+    """Contexts closed with both their graphs captured give the device's memory back (a graph holds some 150 KB, 44 MB in
+    all; the driver takes memory in pieces, so some of that may stay)."""
     import torch
     m = ks.PolarizedSplats(torch.tensor(wide_splats(3, 36), device="cuda"))
 
@@ -321,9 +322,9 @@ def test_a_closed_context_leaves_no_graph():
     for _ in range(3):
         one()
     before = torch.cuda.mem_get_info()[0]
-    for _ in range(60):
+    for _ in range(300):
         one()
-    assert before - torch.cuda.mem_get_info()[0] <= 4 * 2 ** 20
+    assert before - torch.cuda.mem_get_info()[0] <= 16 * 2 ** 20
 
 
 @pytest.mark.parametrize("kappa", [3.05, 7.0, 12.0, 25.0])
