@@ -36,7 +36,7 @@ struct DevBuf {
 };
 
 struct ks_context {
-    int device = 0;
+    int device = 0, nsm = 0;
     cudaStream_t stream = nullptr;
     std::string err;
     long long npix = 0, npad = 0;

@@ -103,12 +103,12 @@ static Shape transport_shape(int ntot, int nkv, int seg_len, int maxb) {
 }
 
 template <class T, int CH, int KM, int NT, int MINB>
-static int run_transport(ks_context* c, TransportJob job, const Shape& sh, int nsm, T* stream, T* seg_out, long long nout) {
+static int run_transport(ks_context* c, TransportJob job, const Shape& sh, T* stream, T* seg_out, long long nout) {
     auto* kernel = k_transport<T, CH, KM, NT, MINB>;
     KS_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sh.smem)));
     job.run = sh.run; job.cap = sh.cap; job.rows_shared = sh.rows_shared ? 1 : 0;
     const long long total = job.nchunks * job.nseg * job.nframes * job.nvc;
-    const long long grid = std::min<long long>(total, (long long)nsm * sh.blocks);
+    const long long grid = std::min<long long>(total, (long long)c->nsm * sh.blocks);
     const double* dt = c->combos.as<double>();
     KS_CUDA(c, cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long), c->stream));
     kernel<<<unsigned(grid), NT, sh.smem, c->stream>>>(plan_view(c), c->st, job, c->rows.as<T>(), dt, dt + job.nframes, stream,
@@ -158,8 +158,6 @@ static TransportJob transport_job(ks_context* c, int ntot, int nframes, int nfre
 template <int CH, int KM>
 static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long npad,
                     float* gstate, unsigned char* gact) {
-    int nsm = 0;
-    KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     // one march per ray, shared by every frame and frequency
     int s = mixed_stream(c, j0, m, npad);
     if (s || (s = build_rows<float, KM>(c, ntot, gstate != nullptr))) return s;
@@ -179,7 +177,7 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     bool wide = s256.blocks * 8 > s128.blocks * 4;
     if (c->tune_nt == 256 && s256.blocks > 0) wide = true;
     if (c->tune_nt == 128 && s128.blocks > 0) wide = false;
-    segment(job, c->st.N, (long long)nsm * (wide ? s256.blocks : s128.blocks), c->tune_units > 0 ? c->tune_units : 8);
+    segment(job, c->st.N, (long long)c->nsm * (wide ? s256.blocks : s128.blocks), c->tune_units > 0 ? c->tune_units : 8);
     // runs no longer than a segment
     if (wide) s256 = transport_shape<float, CH, KM, 256>(ntot, c->nkv, job.seg_len, B256);
     else s128 = transport_shape<float, CH, KM, 128>(ntot, c->nkv, job.seg_len, B128);
@@ -189,8 +187,8 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     KS_CUDA(c, c->seg_out.ensure(size_t(nframes) * nfreq * job.nseg * m * 20 * sizeof(float)));
     KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));   // the adjoint's two counters: no move under a captured render
     if (!c->capturing) cudaEventRecord(c->evc0, c->stream);
-    s = wide ? run_transport<float, CH, KM, 256, B256>(c, job, s256, nsm, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix)
-             : run_transport<float, CH, KM, 128, B128>(c, job, s128, nsm, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix);
+    s = wide ? run_transport<float, CH, KM, 256, B256>(c, job, s256, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix)
+             : run_transport<float, CH, KM, 128, B128>(c, job, s128, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix);
     if (!c->capturing) {
         cudaEventRecord(c->evc1, c->stream);
         c->consume_timed = true;
@@ -218,8 +216,6 @@ int launch_mixed(ks_context* c, int ntot, int nframes, int nfreq, double L, int 
 template <int KM>
 static int plain_piece(ks_context* c, int ntot, int nframes, int nfreq, double L, int nmax, double slab, long long j0, long long m, long long npad,
                        double* gstate, unsigned char* gact) {
-    int nsm = 0;
-    KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     const int N = c->st.N;
     KS_CUDA(c, c->stream64.ensure(size_t(npad) * N * SM_COUNT * sizeof(double)));
     KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));
@@ -237,12 +233,12 @@ static int plain_piece(ks_context* c, int ntot, int nframes, int nfreq, double L
     constexpr int B = 2;
     Shape sh = transport_shape<double, 1, KM, 128>(ntot, c->nkv, N, B);
     if (sh.blocks == 0) return fail(c, KS_ERR_ARGUMENT, "too many splats for one launch (%d)", ntot);
-    segment(job, N, (long long)nsm * sh.blocks, 8);
+    segment(job, N, (long long)c->nsm * sh.blocks, 8);
     sh = transport_shape<double, 1, KM, 128>(ntot, c->nkv, job.seg_len, B);
     job.gstate = gstate; job.gact = gact;
     if (gstate) c->last_job = job;
     KS_CUDA(c, c->seg_out64.ensure(size_t(nframes) * nfreq * job.nseg * m * 20 * sizeof(double)));
-    return run_transport<double, 1, KM, 128, B>(c, job, sh, nsm, stream, c->seg_out64.as<double>(), c->npix);
+    return run_transport<double, 1, KM, 128, B>(c, job, sh, stream, c->seg_out64.as<double>(), c->npix);
 }
 
 static int clear_residuals(ks_context* c) {

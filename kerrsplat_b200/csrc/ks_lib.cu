@@ -561,9 +561,9 @@ __global__ void k_thin_sum(long long npix, int nseg, const double* __restrict__ 
 }
 
 // Pieces of a screen's depth: until there are four blocks per SM, down to one re-anchoring interval each (up to 16).
-int thin_pieces(const Spacetime& st, long long npix) {
+int thin_pieces(const Spacetime& st, long long npix, int nsm) {
     int nseg = 1;
-    while (nseg < 16 && (npix + 31) / 32 * nseg < 4 * 148 && 2 * nseg * (long long)st.M <= st.N) nseg *= 2;
+    while (nseg < 16 && (npix + 31) / 32 * nseg < 4 * nsm && 2 * nseg * (long long)st.M <= st.N) nseg *= 2;
     return nseg;
 }
 
@@ -928,7 +928,7 @@ int check_device_flag(ks_context* c, const char* what) {
 // Allocates nothing: the pieces' sums have their place since regenerate.
 template <class T>
 int launch_thin(ks_context* c, const double* tab, int nsplat, double t_obs, const long long* perm, double* out, bool resid) {
-    const int nseg = thin_pieces(c->st, c->npix);
+    const int nseg = thin_pieces(c->st, c->npix, c->nsm);
     const size_t smem = (sizeof(MarchShared<T>) + 15) / 16 * 16 + size_t(nsplat) * kThinRow * sizeof(T);
     double* rt = resid ? c->resid_t.as<double>() : nullptr;
     double* rp = resid ? c->resid_phi.as<double>() : nullptr;
@@ -975,6 +975,7 @@ int ks_context_create(int device, int flags, ks_context** out) {
     if (cudaSetDevice(device) != cudaSuccess) return KS_ERR_DEVICE;
     ks_context* c = new ks_context();
     c->device = device;
+    if (cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) { delete c; return KS_ERR_DEVICE; }
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return KS_ERR_DEVICE; }
     cudaEventCreate(&c->ev0);
     cudaEventCreate(&c->ev1);
@@ -1199,7 +1200,7 @@ int regenerate_impl(ks_context* c, double a, double theta_o, int32_t nsamples, i
     c->launches++;
     KS_CUDA(c, cudaGetLastError());
     KS_CUDA(c, c->resid_t.ensure(n * sizeof(double)));
-    if (thin_pieces(st, n) > 1) KS_CUDA(c, c->thin_part.ensure(3 * size_t(thin_pieces(st, n)) * n * sizeof(double)));
+    if (const int pieces = thin_pieces(st, n, c->nsm); pieces > 1) KS_CUDA(c, c->thin_part.ensure(3 * size_t(pieces) * n * sizeof(double)));
     KS_CUDA(c, c->resid_phi.ensure(n * sizeof(double)));
     KS_CUDA(c, cudaMemsetAsync(c->resid_t.p, 0, n * sizeof(double), c->stream));
     KS_CUDA(c, cudaMemsetAsync(c->resid_phi.p, 0, n * sizeof(double), c->stream));
@@ -1908,7 +1909,7 @@ int jvp_chunk(ks_context* c, int ntot, const double* dparams_dev, const double* 
     if constexpr (std::is_same<S, float>::value) {
         // segments until there are some 32 warps per SM (at least 16 samples each), as far as 4 GB of segment states go
         int nseg = 1;
-        while (nrc * nseg < 148LL * 1024 && (nseg * 2) * 16 <= c->st.N && nrc * nseg * 2 * 20 * (K + 1) * (long long)sizeof(float) <= (4LL << 30)) nseg *= 2;
+        while (nrc * nseg < c->nsm * 1024LL && (nseg * 2) * 16 <= c->st.N && nrc * nseg * 2 * 20 * (K + 1) * (long long)sizeof(float) <= (4LL << 30)) nseg *= 2;
         // fewer where memory runs out
         for (;; nseg /= 2) {
             const cudaError_t e = c->jvp_part.ensure(size_t(nrc) * nseg * 20 * (K + 1) * sizeof(float));

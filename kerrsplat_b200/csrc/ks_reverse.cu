@@ -17,8 +17,6 @@ template <class T, int CH, int NT, int MINB>
 static int reverse_ch(ks_context* c, int ntot, int nmax, bool add) {
     using SM = ReverseSmem<T, CH, NT>;
     constexpr bool plain = sizeof(T) == 8;
-    int nsm = 0;
-    KS_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     TransportJob job = c->last_job;
     job.kstop = nmax >= 0 ? c->kstop.as<int>() : nullptr;
     // as many blocks as fit (registers hold MINB) with a full window each; the longest run, then the most records; rows
@@ -53,7 +51,7 @@ static int reverse_ch(ks_context* c, int ntot, int nmax, bool add) {
     KS_CUDA(c, c->adj_unit.ensure(size_t(total) * gsz * sizeof(T)));
     KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));
     KS_CUDA(c, cudaMemsetAsync(c->work.p, 0, 2 * sizeof(unsigned long long), c->stream));
-    const long long grid = std::min<long long>(total, (long long)nsm * std::max(per_sm, 1));
+    const long long grid = std::min<long long>(total, (long long)c->nsm * std::max(per_sm, 1));
     kernel<<<unsigned(grid), NT, smem, c->stream>>>(plan_view(c), c->st, job, c->rows.as<T>(), dt, dn, stream, c->adj_bnd.as<T>(),
                                                     c->work.as<unsigned long long>(), c->adj_unit.as<T>(), c->errflag.as<unsigned>());
     const int per_chunk = 256;
