@@ -111,9 +111,15 @@ static int run_transport(ks_context* c, TransportJob job, const Shape& sh, T* st
     const long long grid = std::min<long long>(total, (long long)c->nsm * sh.blocks);
     const double* dt = c->combos.as<double>();
     KS_CUDA(c, cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long), c->stream));
+    const bool timed = sizeof(T) == 4 && !c->capturing;   // ks_consume_stats
+    if (timed) cudaEventRecord(c->evc0, c->stream);
     kernel<<<unsigned(grid), NT, sh.smem, c->stream>>>(plan_view(c), c->st, job, c->rows.as<T>(), dt, dt + job.nframes, stream,
                                                        c->work.as<unsigned long long>(), seg_out,
                                                        c->count_events ? c->counters.as<unsigned long long>() : nullptr, c->errflag.as<unsigned>());
+    if (timed) {
+        cudaEventRecord(c->evc1, c->stream);
+        c->consume_timed = true;
+    }
     c->launches++;
     c->kernel_launches++;
     KS_CUDA(c, cudaGetLastError());
@@ -186,14 +192,8 @@ static int mixed_ch(ks_context* c, int ntot, int nframes, int nfreq, double L, i
     c->last_job = job;   // as the reverse pass walks it
     KS_CUDA(c, c->seg_out.ensure(size_t(nframes) * nfreq * job.nseg * m * 20 * sizeof(float)));
     KS_CUDA(c, c->work.ensure(2 * sizeof(unsigned long long)));   // the adjoint's two counters: no move under a captured render
-    if (!c->capturing) cudaEventRecord(c->evc0, c->stream);
-    s = wide ? run_transport<float, CH, KM, 256, B256>(c, job, s256, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix)
-             : run_transport<float, CH, KM, 128, B128>(c, job, s128, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix);
-    if (!c->capturing) {
-        cudaEventRecord(c->evc1, c->stream);
-        c->consume_timed = true;
-    }
-    return s;
+    return wide ? run_transport<float, CH, KM, 256, B256>(c, job, s256, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix)
+                : run_transport<float, CH, KM, 128, B128>(c, job, s128, c->stream_buf.as<float>(), c->seg_out.as<float>(), c->npix);
 }
 
 // Up to four frequencies share a unit's march, tests and frames.
