@@ -246,7 +246,7 @@ def run_ours(args):
                    "l2": "no flush: the per-ray FP64 plan + anchor table (~150 MB) exceeds the 126 MB L2"},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
-                     "traffic": traffic, "traffic_source": "ncu DRAM bytes of one k_transport launch of this workload (256x256, N=1024, 3 frequencies)"
+                     "traffic": traffic, "traffic_source": "ncu DRAM bytes of one k_transport launch on a scene of this workload's size (256x256, N=1024, 3 frequencies)"
                      if traffic else None,
                      "peak_source": "nominal FP32 pipe (148 SMs x 128 lanes x 2 x max SM clock); MEASURED_PEAKS.json has no FP32 figure",
                      "kernel": kname, "kernel_ms": launch_ms, "flops_per_launch": flops_per_launch,

@@ -12,6 +12,10 @@
  *     host arrays are staged through the library's own device buffers;
  *   - the library owns the per-ray constants, the anchor table and its scratch buffers; the
  *     caller owns inputs and outputs;
+ *   - scratch buffers keep the largest size that a call needed until ks_context_destroy. The large
+ *     ones: the FP32 stream, 32 bytes a (sample, ray); the FP32 gradient's state, 113 bytes a
+ *     (combination, sample, ray); in FP64 at most 4 GB of stream, 4 GB of segment states and 24 GB of
+ *     state, the rays in pieces. Where they do not fit, gradients and FP64 renders take smaller pieces;
  *   - a context is not thread-safe: one context per host thread, or external locking.
  *
  * Each declaration cites the reference (KerrSplat.jl) entry point it replaces, by file:line
@@ -36,7 +40,7 @@ extern "C" {
 #define KS_ERR_TIMEOUT 6          /* a bounded device wait gave up */
 
 /* precision of a render */
-#define KS_FP64 0   /* the plain FP64 path: one re-march per (frame, frequency), like the reference */
+#define KS_FP64 0   /* the plain FP64 path: FP64 throughout, the march once per render */
 #define KS_MIXED 1  /* FP64 ray constants and anchors; the march once per render in FP32 (the radial
                        recurrence and the quadrature, re-anchored to the FP64 anchors every M samples;
                        the polar state, cos theta and krang_visible in FP64); the FP32 transport
@@ -164,9 +168,10 @@ int ks_frame_chi2_seed(ks_context* ctx, const double* image, int32_t order, int6
  * sweep_passes, src/Fit/Fit.jl:451-485). Thermal polarized splats (KS_THERMAL21) only, as in the
  * reference. dstokes has the layout of ks_render's out (npix x 4 x nframes x nfreq, pixels in
  * `order`), the adjoint of the observed Stokes vectors in cgs. dparams receives 21 x nsplat per set,
- * column-major, the sets concatenated; with `accumulate` the gradient is added to it. KS_FP64 runs
- * the reference's structure (stored FP64 samples, backward tails, forward duals, per-ray slots);
- * KS_MIXED the FP32 transport with a per-segment reverse pass. Deterministic: no atomics. */
+ * column-major, the sets concatenated; with `accumulate` the gradient is added to it. Both precisions
+ * run a forward pass that leaves its state at every active sample and a reverse pass over it in work
+ * units, KS_MIXED in FP32. Deterministic: every unit has its own sums, added in a fixed order. A call
+ * whose kernels give up (KS_ERR_TIMEOUT) leaves dparams as it was. */
 int ks_adjoint(ks_context* ctx, const ks_splat_set* sets, int32_t nsets, const double* times, int32_t nframes, const double* nus,
                int32_t nfreq, double L, int32_t precision, int32_t nmax, double slab, const double* dstokes, int32_t order,
                double* dparams, int32_t accumulate);
@@ -231,9 +236,9 @@ int ks_normal_matrix(ks_context* ctx, const double* J, int64_t m, int64_t n, int
 /* sample_adjoint (src/Transfer/transport.jl:221-245) of n independent samples in FP64: for the summed
  * coefficients in (j 4, alpha 4, rho 3 per sample), the step length Dl, the adjoint w in front of the
  * sample and the tail R behind it, out[31 i ..] = O (16, row-major), E (4) and c-bar = (j-bar 4,
- * alpha-bar 4, rho-bar 3), the partials of w^T (O R + E). method 0: the structured form of the mixed
- * path's reverse pass; 1: seven forward-mode duals through the step operator (the reference's form,
- * used by the FP64 adjoint). Arrays host or device. */
+ * alpha-bar 4, rho-bar 3), the partials of w^T (O R + E). method 0: the structured form of the reverse
+ * pass; 1: seven forward-mode duals through the step operator (the reference's form, a check on the
+ * other). Arrays host or device. */
 int ks_sample_adjoint(ks_context* ctx, int64_t n, const double* in, const double* Dl, const double* w, const double* R, int32_t method,
                       double* out);
 
@@ -248,11 +253,11 @@ int ks_kernel_stats(ks_context* ctx, double* render_ms, long long* render_launch
 
 /* CUDA graph of one mixed render (the fit loop's forward pass with no host work): records the device
  * work of ks_render(..., KS_MIXED, ...) for device-resident splat sets (params, and hyp of kappa sets,
- * in device memory) and a device `out`: the splat tables built from the parameters, their FP32 copy,
- * the sample stream, the consumer, the segment composition and the output in `order`. The call first
+ * in device memory) and a device `out`: the splat tables built from the parameters, the sample stream,
+ * the transport, the segment composition and the output in `order`. The call first
  * renders once the ordinary way (validation, buffers, launch shape). Frames, frequencies, L, nmax,
- * slab, the knot array, the splat counts and all pointers are fixed at capture; every replay re-reads
- * the parameter values, so updating them in place on the device and replaying re-renders. One graph
+ * slab, the knot array, the splat counts and all pointers are fixed at capture (the graph keeps its own
+ * copies of the first and of the knots); every replay re-reads the parameter values, so updating them in place on the device and replaying re-renders. One graph
  * per context; a new capture or ks_graph_destroy releases the previous one. */
 int ks_render_graph_capture(ks_context* ctx, const ks_splat_set* sets, int32_t nsets, const double* times, int32_t nframes,
                             const double* nus, int32_t nfreq, double L, int32_t nmax, double slab, double* out, int32_t order);
@@ -283,15 +288,15 @@ int ks_chi2_gradient_graph_launch(ks_context* ctx, int32_t wait);
 /* Release the captured graphs (the render's and the chi^2 + gradient evaluation's). */
 int ks_graph_destroy(ks_context* ctx);
 
-/* Test hook for the bounded waits (no reference counterpart): while on != 0, the transport and
- * reverse kernels of either precision arm the shared-memory barrier of their splat-table staging without issuing the copy and poll it only
- * 4096 times, and the tcgen05 GEMM arms its operand barriers without issuing the tile copies and gives
- * each wait ~10 ms, so every block's wait runs out; the kernels record it, free what they hold and
- * return (no fault, no hang) and the call fails with KS_ERR_TIMEOUT. The context stays usable; turn
- * the hook off to render again. */
+/* Test hook for the bounded waits (no reference counterpart): while on != 0, the transport and reverse
+ * kernels of either precision arm the shared-memory barrier of their splat-table staging without
+ * issuing the copy and poll it only 4096 times, and the tcgen05 GEMM arms its operand barriers without
+ * issuing the tile copies and gives each wait ~10 ms, so every block's wait runs out; the kernels
+ * record it, free what they hold and return (no fault, no hang) and the call fails with
+ * KS_ERR_TIMEOUT. The context stays usable; turn the hook off to render again. */
 int ks_set_stage_test(ks_context* ctx, int32_t on);
 
-/* Device time (CUDA events on the context stream) of the persistent consumer k_transport alone in the
+/* Device time (CUDA events on the context stream) of the transport kernel k_transport alone in the
  * mixed ks_render calls since the last reset, and its launch count (one per mixed render). */
 int ks_consume_stats(ks_context* ctx, double* consume_ms, long long* launches, int reset);
 
@@ -300,8 +305,8 @@ int ks_consume_stats(ks_context* ctx, double* consume_ms, long long* launches, i
 int ks_adjoint_stats(ks_context* ctx, double* adjoint_ms, long long* launches, int reset);
 
 /* The autotuner of the mixed forward pass: renders the scene (mixed precision) with every block size
- * (384, 256, 128 threads of the persistent consumer, where it fits) and work-unit density (2, 4, 8 or 16
- * work units per resident warp, which sets how finely rays are split into sample segments), `trials`
+ * (256, 128 threads of the transport kernel, where it fits) and work-unit density (2, 4, 8 or 16
+ * work units per resident block, which sets how finely rays are split into sample segments), `trials`
  * timed renders each after one warm-up, and keeps the fastest for this context's later calls; block,
  * units and best_ms (the render kernels' time) report the choice. */
 int ks_autotune(ks_context* ctx, const ks_splat_set* sets, int32_t nsets, const double* times, int32_t nframes, const double* nus,

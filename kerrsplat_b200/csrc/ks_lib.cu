@@ -1035,7 +1035,7 @@ int ks_kernel_stats(ks_context* c, double* render_ms, long long* render_launches
     return KS_OK;
 }
 
-// Test hook of the staging error path: while on, the mixed kernels arm their table-staging barrier
+// Test hook of the staging error path: while on, the transport and reverse kernels arm their table-staging barrier
 // without issuing the copy, so the bounded wait runs out and the call fails with KS_ERR_TIMEOUT.
 int ks_set_stage_test(ks_context* c, int32_t on) {
     if (!c) return KS_ERR_ARGUMENT;

@@ -1,4 +1,4 @@
-// ks_reverse.cu -- the mixed reverse pass (ks_reverse.cuh): its launches and the reduction into parameter rows.
+// ks_reverse.cu -- the reverse pass (ks_reverse.cuh): its launches and the reduction into parameter rows.
 #include <algorithm>
 
 #include "../../include/kerrsplat_b200.h"

@@ -1,4 +1,4 @@
-// ks_reverse.cuh -- the mixed reverse pass of the polarized transport: the gradient of sum(dstokes * Stokes) in every
+// ks_reverse.cuh -- the reverse pass of the polarized transport, in FP32 or FP64: the gradient of sum(dstokes * Stokes) in every
 // parameter of the thermal splats (the reference's dual sweep, src/Splats/dual_gradient.jl).
 //
 // The forward pass (k_transport with a gstate) leaves, at every active (sample, ray, frequency), the state P of the
@@ -18,7 +18,7 @@
 // and turned into parameter rows once, in FP64. Each splat's sums of a window are formed by one warp in a fixed
 // order and every unit has its own block of partial sums, so the gradient is the same bit for bit.
 //
-// Bound by instruction issue (41% of the issue slots at 12 warps per SM, its registers' limit). 224 x 224 x 896, 64 splats,
+// Bound by instruction issue (44% of the issue slots at 12 warps per SM, its registers' limit). 224 x 224 x 896, 64 splats,
 // three frequencies: 11.1 ms; the step and element kernels before it took 28.7 ms. Four blocks per SM (128 registers) spill:
 // the whole gradient 23.6 ms against 22.5.
 #pragma once

@@ -72,8 +72,8 @@ def test_transport_edges(oracle, na, nb, N, ns, nf, nmax):
 
 @pytest.mark.parametrize("shift", [-12.0, -4.0, 0.0, 2.0])
 def test_step_adjoint_strengths(shift):
-    """The FP32 step adjoint on weak steps (its power series) and strong ones (its FP64 partials): electron densities
-    e^shift apart put the squared strength of a step below, across and above 1/8."""
+    """The FP32 gradient over electron densities e^shift apart, thin to thick. (test_gpu_device_functions.py runs the step
+    adjoint by itself on both sides of its switch.)"""
     cam = ks.Camera((-8.9, 9.3), (-9.1, 8.7), (17, 15))
     cache, p = cache_of(cam, 96), wide_splats(12, 8)
     p[12] += shift
