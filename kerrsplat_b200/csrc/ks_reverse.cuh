@@ -144,11 +144,9 @@ __device__ __forceinline__ void thermal_row_bar(const T* r, T ne, T nu, T st, T 
     const T ry = y + y * hrcp(em1);                              // d ln(1 / B) / d ln y
     // the cap (coefficients.jl:264-288): jQ, jV scaled by 0.99 jI / sqrt(jQ^2 + jV^2) where that is below one
     T cap = T(1), qq = T(0), vv = T(0), ip2 = T(0);              // ip2 != 0: capped; jQ / jI, jV / jI, 1 / (their squares' sum)
-    if (jI > T(0)) {
-        T I = jI, Q = jQ, V = jV;
-        scale_small(I, Q, V);
-        const T iI = hrcp(I);
-        qq = Q * iI; vv = V * iI;
+    if (jI > T(0)) {   // the ratios of the fits, as thermal_row takes them
+        const T iI = hrcp(fI);
+        qq = fQ * iI; vv = T(4.0 / 3 / 2.5651) * iT * ist * ct * fV * iI;
         const T p2 = qq * qq + vv * vv;
         if (p2 > T(0.9801)) {
             cap = T(0.99) * hrsqrt(p2);

@@ -281,21 +281,22 @@ __device__ __forceinline__ LFrame<T> row_frame(const SampleFrame<T>& F, const T*
 // The smallest normal number: below it the hardware reciprocal is infinite.
 template <class T> __device__ __forceinline__ constexpr T smallest() { return sizeof(T) == 4 ? T(1.17549435e-38) : T(2.2250738585072014e-308); }
 
-// A coefficient below the smallest normal number and those it is compared with, scaled by a power of two into range.
+// cap_factor (coefficients.jl:264-288) from the ratios of Q and V to I
 template <class T>
-__device__ __forceinline__ void scale_small(T& I, T& Q, T& V) {
-    if (I >= smallest<T>()) return;
-    const T b = sizeof(T) == 4 ? T(18446744073709551616.0) : T(1.3407807929942597e154);   // 2^64, 2^512
-    I *= b; Q *= b; V *= b;
+__device__ __forceinline__ T ratio_cap(T q, T v) {
+    const T p2 = q * q + v * v;
+    return p2 > T(0.9801) ? T(0.99) * hrsqrt(p2) : T(1);
 }
-
-// cap_factor (coefficients.jl:264-288) from the ratios to the intensity's coefficient
+// ... from the coefficients; those below the smallest normal number scaled by a power of two into range
 template <class T>
 __device__ __forceinline__ T row_cap(T I, T Q, T V) {
     if (!(I > T(0))) return (Q == T(0) && V == T(0)) ? T(1) : T(0);
-    scale_small(I, Q, V);
-    const T i = hrcp(I), q = Q * i, v = V * i, p2 = q * q + v * v;
-    return p2 > T(0.9801) ? T(0.99) * hrsqrt(p2) : T(1);
+    if (!(I >= smallest<T>())) {
+        const T b = sizeof(T) == 4 ? T(18446744073709551616.0) : T(1.3407807929942597e154);   // 2^64, 2^512
+        I *= b; Q *= b; V *= b;
+    }
+    const T i = hrcp(I);
+    return ratio_cap(Q * i, V * i);
 }
 
 // 1 / B_nu from exp(h nu / k T) - 1; zero where that, or its product with what follows, would overflow: a splat far too
@@ -338,9 +339,11 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     const T e13 = hexp(T(-1.8899) * hexp2(ls));
     constexpr double kJ = kEE * kEE / (2.0 * 1.7320508075688772 * kCL);   // times nu first: 2e-30 n_e underflows in FP32
     const T iT = hrcp(Te), pj = T(kJ) * nu * ne * iT * iT * e13;
-    const T jI = pj * T(2.5651) * (T(1) + T(1.92) * c13 + T(0.9977) * c23);
-    const T jQ = pj * T(2.5651) * (T(1) + T(0.93193) * c13 + T(0.499873) * c23);
-    const T jV = pj * T(4.0 / 3) * iT * ct * hrcp(st) * (T(1.81384) * nus * inu + T(3.42319) * c23 + T(0.0292545) * hexp2(T(-1.5) * ls) + T(2.03773) * c13);
+    // j = pj f: the cap's ratios are the fits' own, whatever range pj is in
+    const T fI = T(2.5651) * (T(1) + T(1.92) * c13 + T(0.9977) * c23);
+    const T fQ = T(2.5651) * (T(1) + T(0.93193) * c13 + T(0.499873) * c23);
+    const T fV = T(4.0 / 3) * iT * ct * hrcp(st) * (T(1.81384) * nus * inu + T(3.42319) * c23 + T(0.0292545) * hexp2(T(-1.5) * ls) + T(2.03773) * c13);
+    const T jI = pj * fI, jQ = pj * fQ, jV = pj * fV, iI = hrcp(fI);
     // 1 / B_nu (planck): the series of exp(y) - 1 below 2e-3
     constexpr double kY = kHPL / (kME * kCL * kCL), kB = 2.0 * kHPL / (kCL * kCL);
     const T y = T(kY) * nu * iT;
@@ -349,7 +352,7 @@ __device__ __forceinline__ bool thermal_row(const T* r, T ne, T nu, T st, T ct, 
     else if constexpr (sizeof(T) == 4) em1 = expm1f(y);
     else em1 = expm1(y);
     const T iB = planck_inverse(T(kB * 1e33), nu, em1);
-    const T cap = row_cap(jI, jQ, jV);
+    const T cap = ratio_cap(fQ * iI, fV * iI);
     c[0] = jI; c[1] = jQ * cap; c[2] = jV * cap;
     c[3] = jI * iB; c[4] = c[1] * iB; c[5] = c[2] * iB;
     return jI > T(0) || c[6] != T(0) || c[7] != T(0);
