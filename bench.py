@@ -338,7 +338,7 @@ def chi2_grad_bench(args, cache, c, dev, stream, world):
     except Exception as exc:   # reported, not fatal
         out["graph"] = {"error": str(exc)}
     if args.fp64_steps > 0:
-        step(ks.KS_FP64)   # stored samples are built on the first FP64 call after a regenerate
+        step(ks.KS_FP64)   # the first FP64 call allocates its stream and state
         torch.cuda.synchronize(dev)
         e0.record(stream)
         for _ in range(args.fp64_steps):

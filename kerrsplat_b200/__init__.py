@@ -81,7 +81,7 @@ class Camera:
 
 
 class Fused:
-    """Fused(M): the march runs inside the consumer, re-anchored every M samples (cache.jl:57-61)."""
+    """Fused(M): the march runs with the render that consumes it, re-anchored every M samples (cache.jl:57-61)."""
 
     def __init__(self, M=64):
         self.M = int(M)

@@ -385,11 +385,9 @@ def test_mixed_adjoint_large_splat_table():
 
 
 def _crowded_scene():
-    """480 wide splats (6 M) stacked on one spot (the FP64 plain adjoint stages at most 501): every
-    sample near it passes every splat, so a block of the mixed kernels collects 384 x 256 pairs for a
-    group of candidate words (past its pair list: the group is redone chunk by chunk) and 384 x 32 for
-    one chunk (past it again: the chunk's list goes in two windows). The second block unit of the
-    24 x 24 screen has dead warps."""
+    """480 wide splats (6 M) stacked on one spot (the FP64 plain adjoint takes at most 501): every sample
+    near it passes every splat, so all fifteen mask words of a sample are full, a sample has more splats
+    than the sort of a window tells apart (32), and the records of a run go in several windows."""
     c = scenes.config2(res=24, N=64)
     rng = np.random.Generator(np.random.PCG64(33))
     p = scenes.thermal_params(rng, 480, c["a"], rlo=5.5, rhi=6.5)
@@ -403,8 +401,8 @@ def _crowded_scene():
 
 
 def test_crowded_pair_lists():
-    """The mixed forward pass and chi^2 gradient on the crowded scene: the chunk-by-chunk and windowed
-    pair lists give the FP64 plain results (image 1e-4, chi^2 1e-3, gradient 1e-3 rel L2)."""
+    """The mixed forward pass and chi^2 gradient on the crowded scene: full masks and several windows a
+    run give the FP64 plain results (image 1e-4, chi^2 1e-3, gradient 1e-3 rel L2)."""
     c, p, cache = _crowded_scene()
     m = ks.PolarizedSplats(p)
     nus = [230e9]
